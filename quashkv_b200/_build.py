@@ -1,7 +1,8 @@
-"""In-tree build of ``libquashkv_b200.so`` (nvcc, sm_100a only).
+"""In-tree build of ``libquashkv_b200.so`` (nvcc, sm_100a only) and of ``quashkv_host.so`` (g++: the host side of
+the hot ops over torch's C++ API).
 
-``python -m quashkv_b200._build`` or ``build()``; the library lands in
-``quashkv_b200/lib/`` next to the sources so that it travels with the tree.
+``python -m quashkv_b200._build`` or ``build()``; the libraries land in
+``quashkv_b200/lib/`` next to the sources so that they travel with the tree.
 """
 
 from __future__ import annotations
@@ -15,6 +16,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libquashkv_b200.so")
+HOST_PATH = os.path.join(LIB_DIR, "quashkv_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host_ops.cpp")
 SOURCES = ["rotate_quant.cu", "rotate_mma.cu", "rotate_umma.cu", "decompress_umma.cu", "packing.cu", "attention.cu", "attention_mma.cu", "attention_tiled.cu", "tiling.cu", "index_scan.cu", "index_scan_mma.cu", "index_scan_umma.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -43,10 +46,28 @@ def _stale() -> bool:
     return _newer(LIB_PATH, _sources() + _headers())
 
 
+def _build_host() -> None:
+    """The ops' host side, against the headers of the torch that is installed (found without importing it)."""
+    from importlib.util import find_spec
+    torch_dir = os.path.dirname(find_spec("torch").origin)
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    cuda_dir = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{torch_dir}/include",
+           f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{cuda_dir}/include", HOST_SOURCE, "-o", HOST_PATH + ".new",
+           f"-L{torch_dir}/lib", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError("quashkv_b200: g++ failed on host_ops.cpp\n" + proc.stdout + proc.stderr)
+    os.replace(HOST_PATH + ".new", HOST_PATH)       # a process that has the old file loaded keeps it
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile the CUDA sources when the library is missing or older than a source.  Every source becomes an
     object file of its own (compiled side by side, kept under lib/obj so that a change rebuilds one file),
     then the objects are linked into the shared library."""
+    if force or _newer(HOST_PATH, [HOST_SOURCE] + _headers()[-1:]):
+        os.makedirs(LIB_DIR, exist_ok=True)
+        _build_host()
     if not force and not _stale():
         return LIB_PATH
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"

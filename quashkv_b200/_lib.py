@@ -10,7 +10,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from ._build import LIB_PATH
+from ._build import HOST_PATH, LIB_PATH
 
 F32, BF16, F16 = 0, 1, 2
 INDEX_MAX_K = 128
@@ -79,13 +79,35 @@ SIGNATURES = {
 }
 
 _LIB = None
+HOST_READY = False
+
+
+def _path() -> str:
+    return os.environ.get("QUASHKV_B200_LIB", LIB_PATH)
+
+
+def load_host(required: bool = True) -> None:
+    """Register the native implementations of the hot ops (csrc/host_ops.cpp) and point them at the library."""
+    global HOST_READY
+    if HOST_READY or (not required and not (os.path.exists(HOST_PATH) and os.path.exists(_path()))):
+        return
+    lib()
+    if not os.path.exists(HOST_PATH):
+        raise RuntimeError(
+            f"quashkv_b200: {HOST_PATH} not found. Build it with `python -m quashkv_b200._build`; "
+            "there is no fallback implementation.")
+    import torch
+    torch.ops.load_library(HOST_PATH)
+    if C.CDLL(HOST_PATH).quashkv_host_bind(_path().encode()) != 0:
+        raise RuntimeError(f"quashkv_b200: {_path()} lacks an entry point that {HOST_PATH} calls; rebuild both")
+    HOST_READY = True
 
 
 def lib() -> C.CDLL:
     """Load the shared object once; fail loudly if it has not been built."""
     global _LIB
     if _LIB is None:
-        path = os.environ.get("QUASHKV_B200_LIB", LIB_PATH)
+        path = _path()
         if not os.path.exists(path):
             raise RuntimeError(
                 f"quashkv_b200: {path} not found. Build it with `python -m quashkv_b200._build` "

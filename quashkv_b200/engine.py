@@ -66,9 +66,6 @@ class QuashKVEngine:
         self._total_tokens = 0
         self._block_lens: list[int] = []
         self._block_cache = None
-        self._tiled_call = None      # prepared attention call of the decode loop (ops.TiledAttentionCall)
-        self._row_call = None        # ... over row-major planes (ops.RowAttentionCall)
-        self._append_call = None     # prepared compression of new tokens (ops.AppendCall)
 
     # ---- compression ------------------------------------------------------------------------
     def compress_keys(self, keys: torch.Tensor):
@@ -123,35 +120,18 @@ class QuashKVEngine:
         _, v_bounds, _ = vq._on(keys.device)
         b, H, S, _ = keys.shape
         p = self._planes
-        if seg0 == 0 and (b, H) == self._shape:
-            # the usual append over all segments: the prepared call (no op dispatcher, kept staging planes)
-            call = self._append_call
-            if call is None or call.device != keys.device or call.consts[0].data_ptr() != Pi.data_ptr():
-                call = self._append_call = ops.AppendCall(Pi, k_bounds, k_cents, Sgn, kq.mse_bits, v_bounds,
-                                                          self.value_bits)
-            with torch.cuda.device(keys.device):
-                if self._tiled:
-                    call.into_records(keys, values, p["records"], self._row_bytes(), self._capacity, offset)
-                else:
-                    call.into_planes(keys, values, p, offset)
+        consts = (Pi, k_bounds, k_cents, Sgn, kq.mse_bits, v_bounds, self.value_bits)
+        if self._tiled:
+            # packed rows go through a staging area, an exact integer kernel files every token into its record
+            records = p["records"]
+            if (b, H) != self._shape or seg0:
+                records = records[seg0:seg0 + b * H]
+            ops.append_records(keys, values, *consts, records, self._capacity, offset, None)
             return
-        if not self._tiled:
-            sl = slice(seg0, seg0 + b * H)
-            ops.append_kv(keys, values, Pi, k_bounds, k_cents, Sgn, kq.mse_bits, v_bounds, self.value_bits,
-                          p["k_codes"][sl], p["k_signs"][sl], p["k_norms"][sl], p["v_codes"][sl], p["v_norms"][sl],
-                          offset)
-            return
-        # tiled storage: the compress kernels write the reference's packed rows into a dense staging area, an
-        # exact integer kernel files every token into its record
-        pk, ps, pv = self._row_bytes()
-        n = b * H * S
-        u8 = dict(dtype=torch.uint8, device=keys.device)
-        st = (torch.empty((b * H, S, pk), **u8), torch.empty((b * H, S, ps), **u8),
-              torch.empty((b * H, S), dtype=torch.float32, device=keys.device),
-              torch.empty((b * H, S, pv), **u8), torch.empty((b * H, S), dtype=torch.float32, device=keys.device))
-        ops.append_kv(keys, values, Pi, k_bounds, k_cents, Sgn, kq.mse_bits, v_bounds, self.value_bits, *st, 0)
-        assert st[2].numel() == n
-        ops.tile_rows(*st, p["records"][seg0:seg0 + b * H], S, self._capacity, offset, None)
+        planes = (p["k_codes"], p["k_signs"], p["k_norms"], p["v_codes"], p["v_norms"])
+        if (b, H) != self._shape or seg0:
+            planes = [t[seg0:seg0 + b * H] for t in planes]
+        ops.append_kv(keys, values, *consts, *planes, offset)
 
     def append(self, keys: torch.Tensor, values: torch.Tensor) -> None:
         """Compress (batch, heads, seq, head_dim) keys and values and add them to the cache."""
@@ -252,18 +232,11 @@ class QuashKVEngine:
         _, _, v_cents = vq._on(queries.device)
         p = self._planes
         if self._tiled:
-            call = self._tiled_call
-            if call is None or call.device != queries.device or call.consts[0].data_ptr() != Pi.data_ptr():
-                call = self._tiled_call = ops.TiledAttentionCall(Pi, k_cents, v_cents, Sgn, kq.qjl_scale)
-            with torch.cuda.device(queries.device):
-                return call(queries.detach(), p["records"], self._capacity, self._total_tokens, Hkv, float(scale),
-                            bool(causal))
-        call = self._row_call
-        if call is None or call.device != queries.device or call.consts[0].data_ptr() != Pi.data_ptr():
-            call = self._row_call = ops.RowAttentionCall(Pi, k_cents, v_cents, Sgn, kq.qjl_scale, self.key_bits,
-                                                         self.value_bits)
-        with torch.cuda.device(queries.device):
-            return call(queries.detach(), p, self._total_tokens, Hkv, float(scale), bool(causal))
+            return ops.attention_tiled(queries, p["records"], self._capacity, self._total_tokens, Hkv, None, None, 0, Pi,
+                                       k_cents, v_cents, Sgn, kq.qjl_scale, float(scale), bool(causal))
+        return ops.attention(queries, p["k_codes"], p["k_signs"], p["k_norms"], p["v_codes"], p["v_norms"],
+                             self._total_tokens, Hkv, self.key_bits, self.value_bits, Pi, k_cents, v_cents, Sgn,
+                             kq.qjl_scale, float(scale), bool(causal))
 
     def attention_from_host(self, queries_host: torch.Tensor, out_host: torch.Tensor,
                             scale: Optional[float] = None, causal: bool = False) -> torch.cuda.Event:
@@ -335,9 +308,6 @@ class QuashKVEngine:
         kq, vq = self.key_quantizer, self.value_quantizer
         Pi, _, k_cents, Sgn = kq._on(dev)
         _, _, v_cents = vq._on(dev)
-        call = self._tiled_call
-        if call is None or call.device != dev or call.consts[0].data_ptr() != Pi.data_ptr():
-            call = self._tiled_call = ops.TiledAttentionCall(Pi, k_cents, v_cents, Sgn, kq.qjl_scale)
         if scale is None:
             scale = 1.0 / math.sqrt(self.head_dim)
         B, Hq = queries_host.shape[0], queries_host.shape[1]
@@ -354,8 +324,9 @@ class QuashKVEngine:
         ok |= rt.cudaStreamWaitEvent(compute, arrived, 0)
         ok |= rt.cudaStreamWaitEvent(compute, copied, 0)
         with torch.cuda.device(dev):
-            call(slot["q"], self._planes["records"], self._capacity, self._total_tokens, Hkv, float(scale),
-                 bool(causal), out=slot["out"], stream=compute)
+            ops.attention_tiled_out(slot["q"], self._planes["records"], self._capacity, self._total_tokens, Hkv, None,
+                                    None, 0, Pi, k_cents, v_cents, Sgn, kq.qjl_scale, float(scale), bool(causal),
+                                    slot["out"])
         ok |= rt.cudaEventRecord(computed, compute)
         ok |= rt.cudaStreamWaitEvent(d2h, computed, 0)
         ok |= rt.cudaMemcpyAsync(out_host.data_ptr(), slot["out"].data_ptr(), out_host.numel() * 4, 2, d2h)

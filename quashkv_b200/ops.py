@@ -5,6 +5,10 @@ pointers and the current CUDA stream to one ``extern "C"`` entry point, and
 returns.  Only a CUDA implementation is registered: calling an op on CPU
 tensors raises from the dispatcher, there is no fallback.
 
+The ops of the hot paths (schemas below) are implemented in csrc/host_ops.cpp:
+their host side is native.  The others (packing, row scatter, layout changes,
+dense index scores) are Python over ctypes.
+
 Plain Python wrappers of the same names (``ops.compress_mse(...)``) are what the
 host classes call; they normalise shapes and dtypes and then invoke the
 registered op.
@@ -18,7 +22,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import Cache, Rows, TILE_BYTES, TILE_TOKENS, TiledCache
+from ._lib import Rows, TILE_BYTES, TILE_TOKENS
 
 _DT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 
@@ -82,6 +86,42 @@ class _Keep:
         return _p(t)
 
 
+# Ops implemented in csrc/host_ops.cpp.
+_LIBRARY = torch.library.Library("quashkv_b200", "FRAGMENT")
+_CONSTS = "Tensor Pi, Tensor key_centroids, Tensor val_centroids, Tensor S, float qjl_scale, float scale, bool causal"
+_APPEND = ("Tensor keys, Tensor values, Tensor Pi, Tensor k_bounds, Tensor k_cents, Tensor S, int mse_bits, "
+           "Tensor v_bounds, int val_bits")
+_TILED = ("Tensor q, Tensor records, int capacity, int kv_len, int n_kv_heads, Tensor? block_table, Tensor? seq_lens, "
+          f"int block_size, {_CONSTS}")
+for _schema in (
+        "compress_mse(Tensor x, Tensor Pi, Tensor boundaries, int bits, bool packed) -> (Tensor, Tensor)",
+        "compress_ip(Tensor x, Tensor Pi, Tensor boundaries, Tensor centroids, Tensor S, int mse_bits, bool packed) "
+        "-> (Tensor, Tensor, Tensor)",
+        "compress_ip_into(Tensor x, Tensor Pi, Tensor boundaries, Tensor centroids, Tensor S, int mse_bits, "
+        "Tensor(a!) codes, Tensor(b!) signs, Tensor(c!) norms, int offset) -> ()",
+        "compress_mixed(Tensor x, Tensor Pi, Tensor is_outlier, Tensor bounds_out, int bits_out, Tensor bounds_reg, "
+        "int bits_reg, bool packed, int n_out) -> (Tensor, Tensor)",
+        f"append_kv({_APPEND}, Tensor(a!) k_codes, Tensor(b!) k_signs, Tensor(c!) k_norms, Tensor(d!) v_codes, "
+        "Tensor(e!) v_norms, int offset) -> ()",
+        f"append_records({_APPEND}, Tensor(a!) records, int capacity, int offset, Tensor? slots) -> ()",
+        "decompress(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, int bits, Tensor? S, "
+        "float qjl_scale, bool packed, int d, int seg_len, int seg_stride, int seg_off, int n_vec, "
+        "ScalarType out_dtype) -> Tensor",
+        "decompress_mixed(Tensor codes, Tensor norms, Tensor Pi, Tensor is_outlier, Tensor cents_out, int bits_out, "
+        "Tensor cents_reg, int bits_reg, bool packed, int d) -> Tensor",
+        "attention(Tensor q, Tensor k_codes, Tensor k_signs, Tensor k_norms, Tensor v_codes, Tensor v_norms, "
+        f"int kv_len, int n_kv_heads, int key_bits, int val_bits, {_CONSTS}) -> Tensor",
+        "attention_paged(Tensor q, Tensor k_codes, Tensor k_signs, Tensor k_norms, Tensor v_codes, Tensor v_norms, "
+        f"Tensor block_table, Tensor seq_lens, int max_kv_len, int key_bits, int val_bits, {_CONSTS}) -> Tensor",
+        f"attention_tiled({_TILED}) -> Tensor",
+        f"attention_tiled_out({_TILED}, Tensor(a!) out) -> ()",
+        "index_scan_topk(Tensor queries, Tensor db_codes, Tensor db_signs, Tensor db_norms, int n_vectors, int bits, "
+        "Tensor Pi, Tensor centroids, Tensor S, float qjl_scale, int k, int id_base) -> (Tensor, Tensor)"):
+    _LIBRARY.define(_schema)
+_NATIVE = torch.ops.quashkv_b200
+_lib.load_host(required=False)        # not built yet: the first call says so
+
+
 def _flat(x: torch.Tensor):
     d = x.shape[-1]
     if x.dtype not in _DT:
@@ -132,23 +172,7 @@ def _(packed, bits, d):
     return packed.new_empty((*packed.shape[:-1], d))
 
 
-@torch.library.custom_op("quashkv_b200::compress_mse", mutates_args=(), device_types="cuda")
-def _compress_mse(x: torch.Tensor, Pi: torch.Tensor, boundaries: torch.Tensor, bits: int,
-                  packed: bool) -> tuple[torch.Tensor, torch.Tensor]:
-    flat, d = _flat(x)
-    n = flat.shape[0]
-    width = packed_row_bytes(d, bits) if packed else d
-    codes = torch.empty((n, width), dtype=torch.uint8, device=x.device)
-    norms = torch.empty((n,), dtype=torch.float32, device=x.device)
-    A = _Keep(x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().qkv_compress_mse(
-            _p(flat), _DT[flat.dtype], d, n, d, A.f32(Pi), A.f32(boundaries), bits,
-            _p(codes), int(packed), _p(norms), _dense(n), _stream(x)), "compress_mse")
-    return codes.reshape(*x.shape[:-1], width), norms.reshape(x.shape[:-1])
-
-
-@_compress_mse.register_fake
+@torch.library.register_fake("quashkv_b200::compress_mse")
 def _(x, Pi, boundaries, bits, packed):
     d = x.shape[-1]
     width = packed_row_bytes(d, bits) if packed else d
@@ -156,27 +180,7 @@ def _(x, Pi, boundaries, bits, packed):
             x.new_empty(x.shape[:-1], dtype=torch.float32))
 
 
-@torch.library.custom_op("quashkv_b200::compress_ip", mutates_args=(), device_types="cuda")
-def _compress_ip(x: torch.Tensor, Pi: torch.Tensor, boundaries: torch.Tensor, centroids: torch.Tensor,
-                 S: torch.Tensor, mse_bits: int, packed: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    flat, d = _flat(x)
-    n = flat.shape[0]
-    cw = packed_row_bytes(d, mse_bits) if packed else d
-    sw = packed_row_bytes(d, 1) if packed else d
-    codes = torch.empty((n, cw), dtype=torch.uint8, device=x.device)
-    signs = torch.empty((n, sw), dtype=torch.uint8, device=x.device)
-    norms = torch.empty((n,), dtype=torch.float32, device=x.device)
-    A = _Keep(x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().qkv_compress_ip(
-            _p(flat), _DT[flat.dtype], d, n, d, A.f32(Pi), A.f32(boundaries), A.f32(centroids),
-            mse_bits, A.f32(S), _p(codes), _p(signs), int(packed), _p(norms), _dense(n), _stream(x)),
-            "compress_ip")
-    lead = x.shape[:-1]
-    return codes.reshape(*lead, cw), signs.reshape(*lead, sw), norms.reshape(lead)
-
-
-@_compress_ip.register_fake
+@torch.library.register_fake("quashkv_b200::compress_ip")
 def _(x, Pi, boundaries, centroids, S, mse_bits, packed):
     d = x.shape[-1]
     cw = packed_row_bytes(d, mse_bits) if packed else d
@@ -186,70 +190,7 @@ def _(x, Pi, boundaries, centroids, S, mse_bits, packed):
             x.new_empty(x.shape[:-1], dtype=torch.float32))
 
 
-@torch.library.custom_op("quashkv_b200::append_kv", mutates_args=("k_codes", "k_signs", "k_norms", "v_codes", "v_norms"),
-                         device_types="cuda")
-def _append_kv(keys: torch.Tensor, values: torch.Tensor, Pi: torch.Tensor,
-               k_bounds: torch.Tensor, k_cents: torch.Tensor, S: torch.Tensor, mse_bits: int,
-               v_bounds: torch.Tensor, val_bits: int,
-               k_codes: torch.Tensor, k_signs: torch.Tensor, k_norms: torch.Tensor,
-               v_codes: torch.Tensor, v_norms: torch.Tensor, offset: int) -> None:
-    """Compress (B,H,S,d) keys and values straight into the packed cache planes
-    [B*H, capacity, ...] at rows offset..offset+S of every (batch, head) segment."""
-    kf, d = _flat(keys)
-    vf, _ = _flat(values)
-    s_new = keys.shape[-2]
-    cap = k_norms.shape[-1]
-    rows = Rows(s_new, cap, offset)
-    _same_device(keys.device, values, k_codes, k_signs, k_norms, v_codes, v_norms)
-    Pi32 = _f32(Pi, keys.device)
-    A = _Keep(keys.device)
-    with torch.cuda.device(keys.device):
-        L = _lib.lib()
-        _lib.check(L.qkv_compress_ip(
-            _p(kf), _DT[kf.dtype], d, kf.shape[0], d, _p(Pi32), A.f32(k_bounds), A.f32(k_cents), mse_bits,
-            A.f32(S), _p(k_codes), _p(k_signs), 1, _p(k_norms), rows, _stream(keys)), "append keys")
-        _lib.check(L.qkv_compress_mse(
-            _p(vf), _DT[vf.dtype], d, vf.shape[0], d, _p(Pi32), A.f32(v_bounds), val_bits,
-            _p(v_codes), 1, _p(v_norms), rows, _stream(keys)), "append values")
-
-
-@torch.library.custom_op("quashkv_b200::compress_ip_into", mutates_args=("codes", "signs", "norms"),
-                         device_types="cuda")
-def _compress_ip_into(x: torch.Tensor, Pi: torch.Tensor, boundaries: torch.Tensor, centroids: torch.Tensor,
-                      S: torch.Tensor, mse_bits: int, codes: torch.Tensor, signs: torch.Tensor,
-                      norms: torch.Tensor, offset: int) -> None:
-    """Compress (N,d) vectors into packed planes [capacity, bytes] at rows offset..offset+N."""
-    flat, d = _flat(x)
-    n = flat.shape[0]
-    A = _Keep(x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().qkv_compress_ip(
-            _p(flat), _DT[flat.dtype], d, n, d, A.f32(Pi), A.f32(boundaries), A.f32(centroids),
-            mse_bits, A.f32(S), _p(codes), _p(signs), 1, _p(norms), Rows(max(n, 1), 0, offset),
-            _stream(x)), "compress_ip_into")
-
-
-@torch.library.custom_op("quashkv_b200::compress_mixed", mutates_args=(), device_types="cuda")
-def _compress_mixed(x: torch.Tensor, Pi: torch.Tensor, is_outlier: torch.Tensor,
-                    bounds_out: torch.Tensor, bits_out: int, bounds_reg: torch.Tensor, bits_reg: int,
-                    packed: bool, n_out: int) -> tuple[torch.Tensor, torch.Tensor]:
-    """``n_out`` = number of marked channels of ``is_outlier`` (known on the host, so that the packed row width
-    needs no device read)."""
-    flat, d = _flat(x)
-    n = flat.shape[0]
-    width = int(_lib.lib().qkv_mixed_row_bytes(d, n_out, bits_out, bits_reg)) if packed else d
-    codes = torch.empty((n, width), dtype=torch.uint8, device=x.device)
-    norms = torch.empty((n,), dtype=torch.float32, device=x.device)
-    A = _Keep(x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().qkv_compress_mixed(
-            _p(flat), _DT[flat.dtype], d, n, d, A.f32(Pi), A.u8(is_outlier), A.f32(bounds_out), bits_out,
-            A.f32(bounds_reg), bits_reg, _p(codes), int(packed), _p(norms), _dense(n), _stream(x)),
-            "compress_mixed")
-    return codes.reshape(*x.shape[:-1], width), norms.reshape(x.shape[:-1])
-
-
-@_compress_mixed.register_fake
+@torch.library.register_fake("quashkv_b200::compress_mixed")
 def _(x, Pi, is_outlier, bounds_out, bits_out, bounds_reg, bits_reg, packed, n_out):
     d = x.shape[-1]
     width = (n_out * bits_out + 7) // 8 + ((d - n_out) * bits_reg + 7) // 8 if packed else d
@@ -284,119 +225,24 @@ def _(x, Pi, is_outlier, bounds_out, cents_out, bits_out, bounds_reg, cents_reg,
             x.new_empty(x.shape[:-1], dtype=torch.float32))
 
 
-@torch.library.custom_op("quashkv_b200::decompress", mutates_args=(), device_types="cuda")
-def _decompress(codes: torch.Tensor, signs: Optional[torch.Tensor], norms: torch.Tensor, Pi: torch.Tensor,
-                centroids: torch.Tensor, bits: int, S: Optional[torch.Tensor], qjl_scale: float,
-                packed: bool, d: int, seg_len: int, seg_stride: int, seg_off: int, n_vec: int,
-                out_dtype: torch.dtype) -> torch.Tensor:
-    """Rows of the code/norm planes are addressed with (seg_len, seg_stride, seg_off); the
-    output is dense (n_vec, d)."""
-    out = torch.empty((n_vec, d), dtype=out_dtype, device=codes.device)
-    _same_device(codes.device, codes, signs, norms)
-    A = _Keep(codes.device)
-    with torch.cuda.device(codes.device):
-        _lib.check(_lib.lib().qkv_decompress(
-            _p(codes), _p(signs), int(packed), _p(norms), Rows(seg_len, seg_stride, seg_off), n_vec, d,
-            A.f32(Pi), A.f32(centroids), bits, A.f32(S), float(qjl_scale),
-            _p(out), _DT[out_dtype], d, _stream(codes)), "decompress")
-    return out
-
-
-@_decompress.register_fake
+@torch.library.register_fake("quashkv_b200::decompress")
 def _(codes, signs, norms, Pi, centroids, bits, S, qjl_scale, packed, d, seg_len, seg_stride, seg_off,
       n_vec, out_dtype):
     return codes.new_empty((n_vec, d), dtype=out_dtype)
 
 
-@torch.library.custom_op("quashkv_b200::decompress_mixed", mutates_args=(), device_types="cuda")
-def _decompress_mixed(codes: torch.Tensor, norms: torch.Tensor, Pi: torch.Tensor, is_outlier: torch.Tensor,
-                      cents_out: torch.Tensor, bits_out: int, cents_reg: torch.Tensor, bits_reg: int,
-                      packed: bool, d: int) -> torch.Tensor:
-    flat = codes.reshape(-1, codes.shape[-1]).contiguous()
-    n = flat.shape[0]
-    out = torch.empty((n, d), dtype=torch.float32, device=codes.device)
-    _same_device(codes.device, codes, norms)
-    A = _Keep(codes.device)
-    with torch.cuda.device(codes.device):
-        _lib.check(_lib.lib().qkv_decompress_mixed(
-            _p(flat), int(packed), A.f32(norms.reshape(-1)), _dense(n), n, d, A.f32(Pi),
-            A.u8(is_outlier), A.f32(cents_out), bits_out,
-            A.f32(cents_reg), bits_reg, _p(out), _lib.F32, d, _stream(codes)), "decompress_mixed")
-    return out.reshape(*codes.shape[:-1], d)
-
-
-@_decompress_mixed.register_fake
+@torch.library.register_fake("quashkv_b200::decompress_mixed")
 def _(codes, norms, Pi, is_outlier, cents_out, bits_out, cents_reg, bits_reg, packed, d):
     return codes.new_empty((*codes.shape[:-1], d), dtype=torch.float32)
 
 
-@torch.library.custom_op("quashkv_b200::attention", mutates_args=(), device_types="cuda")
-def _attention(q: torch.Tensor, k_codes: torch.Tensor, k_signs: torch.Tensor, k_norms: torch.Tensor,
-               v_codes: torch.Tensor, v_norms: torch.Tensor, kv_len: int, n_kv_heads: int,
-               key_bits: int, val_bits: int, Pi: torch.Tensor, key_centroids: torch.Tensor,
-               val_centroids: torch.Tensor, S: torch.Tensor, qjl_scale: float, scale: float,
-               causal: bool) -> torch.Tensor:
-    """q (B,Hq,Q,d); planes [B*Hkv, capacity, bytes] packed; returns (B,Hq,Q,d) fp32."""
-    B, Hq, Q, d = q.shape
-    if q.dtype not in _DT:
-        q = q.float()
-    qc = q.detach().contiguous()
-    cap = k_norms.shape[-1]
-    out = torch.empty((B, Hq, Q, d), dtype=torch.float32, device=q.device)
-    L = _lib.lib()
-    ws_bytes = L.qkv_attention_workspace_bytes(B, Hq, n_kv_heads, Q, kv_len, d)
-    ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=q.device)
-    _same_device(q.device, k_codes, k_signs, k_norms, v_codes, v_norms)
-    _p(k_codes)                                        # refuses anything that is not device memory
-    cache = Cache(k_codes.data_ptr(), k_signs.data_ptr(), k_norms.data_ptr(), v_codes.data_ptr(),
-                  v_norms.data_ptr(), cap)
-    A = _Keep(q.device)
-    with torch.cuda.device(q.device):
-        _lib.check(L.qkv_attention(
-            _p(qc), _DT[qc.dtype], cache, B, Hq, n_kv_heads, Q, kv_len, d, key_bits, val_bits,
-            A.f32(Pi), A.f32(key_centroids), A.f32(val_centroids), A.f32(S),
-            float(qjl_scale), float(scale), int(causal), _p(out), _p(ws), ws_bytes, _stream(q)), "attention")
-    return out
-
-
-@_attention.register_fake
+@torch.library.register_fake("quashkv_b200::attention")
 def _(q, k_codes, k_signs, k_norms, v_codes, v_norms, kv_len, n_kv_heads, key_bits, val_bits, Pi,
       key_centroids, val_centroids, S, qjl_scale, scale, causal):
     return q.new_empty(q.shape, dtype=torch.float32)
 
 
-@torch.library.custom_op("quashkv_b200::attention_paged", mutates_args=(), device_types="cuda")
-def _attention_paged(q: torch.Tensor, k_codes: torch.Tensor, k_signs: torch.Tensor, k_norms: torch.Tensor,
-                     v_codes: torch.Tensor, v_norms: torch.Tensor, block_table: torch.Tensor,
-                     seq_lens: torch.Tensor, max_kv_len: int, key_bits: int, val_bits: int, Pi: torch.Tensor,
-                     key_centroids: torch.Tensor, val_centroids: torch.Tensor, S: torch.Tensor,
-                     qjl_scale: float, scale: float, causal: bool) -> torch.Tensor:
-    """q (B,Hq,Q,d); pool planes [blocks, Hkv, block_size, bytes] packed; block_table (B, max_blocks) int32;
-    seq_lens (B) int32; max_kv_len an upper bound of seq_lens known on the host.  Returns (B,Hq,Q,d) fp32."""
-    B, Hq, Q, d = q.shape
-    if q.dtype not in _DT:
-        q = q.float()
-    qc = q.detach().contiguous()
-    n_kv_heads, block_size = k_norms.shape[1], k_norms.shape[2]
-    out = torch.empty((B, Hq, Q, d), dtype=torch.float32, device=q.device)
-    L = _lib.lib()
-    ws_bytes = L.qkv_attention_workspace_bytes(B, Hq, n_kv_heads, Q, max_kv_len, d)
-    ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=q.device)
-    _same_device(q.device, k_codes, k_signs, k_norms, v_codes, v_norms, block_table, seq_lens)
-    _p(k_codes)
-    pool = _lib.PagedCache(k_codes.data_ptr(), k_signs.data_ptr(), k_norms.data_ptr(), v_codes.data_ptr(),
-                           v_norms.data_ptr(), block_table.data_ptr(), seq_lens.data_ptr(),
-                           block_table.shape[1], block_size)
-    A = _Keep(q.device)
-    with torch.cuda.device(q.device):
-        _lib.check(L.qkv_attention_paged(
-            _p(qc), _DT[qc.dtype], pool, B, Hq, n_kv_heads, Q, max_kv_len, d, key_bits, val_bits,
-            A.f32(Pi), A.f32(key_centroids), A.f32(val_centroids), A.f32(S),
-            float(qjl_scale), float(scale), int(causal), _p(out), _p(ws), ws_bytes, _stream(q)), "attention_paged")
-    return out
-
-
-@_attention_paged.register_fake
+@torch.library.register_fake("quashkv_b200::attention_paged")
 def _(q, k_codes, k_signs, k_norms, v_codes, v_norms, block_table, seq_lens, max_kv_len, key_bits, val_bits, Pi,
       key_centroids, val_centroids, S, qjl_scale, scale, causal):
     return q.new_empty(q.shape, dtype=torch.float32)
@@ -474,141 +320,6 @@ def _(records, n_rows, seg_len, seg_stride, seg_off, slots):
     return u8(32), u8(16), f32(), u8(48), f32()
 
 
-@torch.library.custom_op("quashkv_b200::attention_tiled", mutates_args=(), device_types="cuda")
-def _attention_tiled(q: torch.Tensor, records: torch.Tensor, capacity: int, kv_len: int, n_kv_heads: int,
-                     block_table: Optional[torch.Tensor], seq_lens: Optional[torch.Tensor], block_size: int,
-                     Pi: torch.Tensor, key_centroids: torch.Tensor, val_centroids: torch.Tensor, S: torch.Tensor,
-                     qjl_scale: float, scale: float, causal: bool) -> torch.Tensor:
-    """q (B,Hq,Q,128); records [B*Hkv, capacity/16, 1664] (contiguous) or [blocks, Hkv, block_size/16, 1664] with a
-    (B, max_blocks) int32 block table and (B) int32 lengths (paged; kv_len is then their host-known upper
-    bound).  Returns (B,Hq,Q,128) fp32.  Pi, centroids and S must be contiguous fp32."""
-    B, Hq, Q, d = q.shape
-    if q.dtype not in _DT:
-        q = q.float()
-    qc = q.detach().contiguous()
-    out = torch.empty((B, Hq, Q, d), dtype=torch.float32, device=q.device)
-    L = _lib.lib()
-    ws_bytes = L.qkv_attention_workspace_bytes(B, Hq, n_kv_heads, Q, kv_len, d)
-    ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=q.device)
-    paged = block_table is not None
-    _same_device(q.device, records, block_table, seq_lens)
-    _p(records)
-    cache = TiledCache(records.data_ptr(), capacity, block_table.data_ptr() if paged else None,
-                       seq_lens.data_ptr() if paged else None, block_table.shape[1] if paged else 0, block_size)
-    Pi32, kc32, vc32, S32 = (_f32(t, q.device) for t in (Pi, key_centroids, val_centroids, S))   # held until the call returns
-    A = _Keep(q.device)
-    with torch.cuda.device(q.device):
-        _lib.check(L.qkv_attention_tiled(
-            _p(qc), _DT[qc.dtype], cache, B, Hq, n_kv_heads, Q, kv_len, d, 3, 3, _p(Pi32), _p(kc32), _p(vc32),
-            _p(S32), float(qjl_scale), float(scale), int(causal), _p(out), _p(ws), ws_bytes, _stream(q)),
-            "attention_tiled")
-    return out
-
-
-class RowAttentionCall:
-    """The C call of the ``attention`` op (row-major packed planes; ``QuashKVEngine.attention``, reference
-    engine.py:204-299), prepared once for an engine's decode loop:
-    constants converted once, the workspace kept and grown when needed, no op dispatcher.  A decode step over a
-    short cache is a few tens of microseconds of device work; the generic op spends more than that on the
-    host.  One instance serves one stream at a time (the workspace is shared by its calls)."""
-
-    def __init__(self, Pi, key_centroids, val_centroids, S, qjl_scale: float, key_bits: int, val_bits: int):
-        self.consts = tuple(_f32(t) for t in (Pi, key_centroids, val_centroids, S))
-        self.ptrs = tuple(_p(t) for t in self.consts)
-        self.qjl_scale, self.key_bits, self.val_bits = float(qjl_scale), int(key_bits), int(val_bits)
-        self.device = self.consts[0].device
-        self.ws = None
-        self.lib = _lib.lib()
-        self.fn = self.lib.qkv_attention
-
-    def __call__(self, q: torch.Tensor, planes: dict, kv_len: int, n_kv_heads: int, scale: float,
-                 causal: bool) -> torch.Tensor:
-        B, Hq, Q, d = q.shape
-        if q.dtype not in _DT:
-            q = q.float()
-        qc = q if q.is_contiguous() else q.contiguous()
-        kn = planes["k_norms"]
-        if qc.device != self.device or kn.device != self.device:
-            raise ValueError(f"quashkv_b200: queries on {qc.device}, planes on {kn.device}, constants on {self.device}")
-        out = torch.empty((B, Hq, Q, d), dtype=torch.float32, device=q.device)
-        need = self.lib.qkv_attention_workspace_bytes(B, Hq, n_kv_heads, Q, kv_len, d)
-        if self.ws is None or self.ws.numel() < need:
-            self.ws = torch.empty((max(need + need // 4, 1 << 16),), dtype=torch.uint8, device=q.device)
-        cache = Cache(planes["k_codes"].data_ptr(), planes["k_signs"].data_ptr(), kn.data_ptr(),
-                      planes["v_codes"].data_ptr(), planes["v_norms"].data_ptr(), kn.shape[-1])
-        rc = self.fn(qc.data_ptr(), _DT[qc.dtype], cache, B, Hq, n_kv_heads, Q, kv_len, d, self.key_bits,
-                     self.val_bits, *self.ptrs, self.qjl_scale, scale, int(causal), out.data_ptr(),
-                     self.ws.data_ptr(), self.ws.numel(), torch.cuda.current_stream(q.device).cuda_stream)
-        if rc:
-            _lib.check(rc, "attention")
-        return out
-
-
-class AppendCall:
-    """Compression of new keys and values into an engine's storage (``QuashKVEngine.append``, reference
-    engine.py:145-172), prepared once: constants converted once,
-    the staging planes of a tiled cache kept between calls, the library called directly.  The generic ops cost
-    80-120 us of host time per one-token append (dispatcher, conversions, five allocations)."""
-
-    def __init__(self, Pi, k_bounds, k_cents, S, mse_bits: int, v_bounds, val_bits: int):
-        self.consts = tuple(_f32(t) for t in (Pi, k_bounds, k_cents, S, v_bounds))
-        self.Pi, self.kb, self.kc, self.S, self.vb = (_p(t) for t in self.consts)
-        self.mse_bits, self.val_bits = int(mse_bits), int(val_bits)
-        self.device = self.consts[0].device
-        self.lib = _lib.lib()
-        self.stage = None           # tiled: (k_codes, k_signs, k_norms, v_codes, v_norms) for up to stage_rows rows
-        self.stage_rows = 0
-        self.stage_stream = None    # the staging planes belong to the stream they were last used on
-
-    def _compress(self, keys, values, ptrs, rows: "Rows", stream) -> None:
-        kf, d = _flat(keys)
-        vf, _ = _flat(values)
-        if kf.device != self.device or vf.device != self.device:
-            raise ValueError(f"quashkv_b200: keys on {kf.device}, constants on {self.device}")
-        L = self.lib
-        rc = L.qkv_compress_ip(kf.data_ptr(), _DT[kf.dtype], d, kf.shape[0], d, self.Pi, self.kb, self.kc,
-                               self.mse_bits, self.S, ptrs[0], ptrs[1], 1, ptrs[2], rows, stream)
-        if rc:
-            _lib.check(rc, "append keys")
-        rc = L.qkv_compress_mse(vf.data_ptr(), _DT[vf.dtype], d, vf.shape[0], d, self.Pi, self.vb, self.val_bits,
-                                ptrs[3], 1, ptrs[4], rows, stream)
-        if rc:
-            _lib.check(rc, "append values")
-
-    def into_planes(self, keys: torch.Tensor, values: torch.Tensor, planes: dict, offset: int) -> None:
-        """(B,H,S,d) keys / values into row-major planes [B*H, capacity, ...] at rows offset..offset+S."""
-        kn = planes["k_norms"]
-        if kn.device != self.device:
-            raise ValueError(f"quashkv_b200: planes on {kn.device}, constants on {self.device}")
-        ptrs = tuple(C.c_void_p(planes[n].data_ptr()) for n in ("k_codes", "k_signs", "k_norms", "v_codes", "v_norms"))
-        self._compress(keys, values, ptrs, Rows(keys.shape[-2], kn.shape[-1], offset),
-                       C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream))
-
-    def into_records(self, keys: torch.Tensor, values: torch.Tensor, records: torch.Tensor, row_bytes: tuple,
-                     capacity: int, offset: int) -> None:
-        """(B,H,S,d) keys / values into tile records [B*H, capacity/16, 1664] at tokens offset..offset+S."""
-        if records.device != self.device:
-            raise ValueError(f"quashkv_b200: records on {records.device}, constants on {self.device}")
-        b, H, S, _ = keys.shape
-        n = b * H * S
-        stream_handle = torch.cuda.current_stream(self.device).cuda_stream
-        if self.stage is None or self.stage_rows < n or self.stage_stream != stream_handle:
-            pk, ps, pv = row_bytes
-            u8 = dict(dtype=torch.uint8, device=self.device)
-            f32 = dict(dtype=torch.float32, device=self.device)
-            self.stage = (torch.empty((n, pk), **u8), torch.empty((n, ps), **u8), torch.empty((n,), **f32),
-                          torch.empty((n, pv), **u8), torch.empty((n,), **f32))
-            self.stage_rows = n
-            self.stage_stream = stream_handle
-        ptrs = tuple(C.c_void_p(t.data_ptr()) for t in self.stage)
-        stream = C.c_void_p(stream_handle)
-        self._compress(keys, values, ptrs, _dense(n), stream)
-        rc = self.lib.qkv_tile_rows(*ptrs, n, C.c_void_p(records.data_ptr()), Rows(max(S, 1), capacity, offset), None,
-                                    stream)
-        if rc:
-            _lib.check(rc, "tile_rows")
-
-
 _CUDART = None
 
 
@@ -629,80 +340,13 @@ def cudart():
     return _CUDART
 
 
-class TiledAttentionCall:
-    """The same C call as the ``attention_tiled`` op (``QuashKVEngine.attention``, reference engine.py:204-299,
-    over a cache kept as tile records), prepared once for an engine's decode loop: constants are
-    converted and kept, the workspace is kept between calls and grows when a longer cache needs more, and the
-    call goes to the library without passing through the op dispatcher.  A decode step over one KV head of a
-    sharded cache lasts tens of microseconds on the device; the per-call host work of the generic op (four
-    tensor conversions, a workspace allocation, the dispatcher) is as long.  One instance serves one stream at
-    a time (the workspace is shared by its calls)."""
-
-    def __init__(self, Pi, key_centroids, val_centroids, S, qjl_scale: float):
-        self.consts = tuple(_f32(t) for t in (Pi, key_centroids, val_centroids, S))
-        self.ptrs = tuple(_p(t) for t in self.consts)
-        self.qjl_scale = float(qjl_scale)
-        self.device = self.consts[0].device
-        self.ws = None
-        self.lib = _lib.lib()
-        self.fn = self.lib.qkv_attention_tiled
-
-    def __call__(self, q: torch.Tensor, records: torch.Tensor, capacity: int, kv_len: int, n_kv_heads: int,
-                 scale: float, causal: bool, out: Optional[torch.Tensor] = None,
-                 stream: Optional[int] = None) -> torch.Tensor:
-        """``out`` (fp32, contiguous, shape of q) is written when given; ``stream`` is a raw stream handle
-        (default: the current stream of q's device)."""
-        B, Hq, Q, d = q.shape
-        if q.dtype not in _DT:
-            q = q.float()
-        qc = q if q.is_contiguous() else q.contiguous()
-        if qc.device != self.device or records.device != self.device:
-            raise ValueError(f"quashkv_b200: queries on {qc.device}, records on {records.device}, constants on {self.device}")
-        if out is None:
-            out = torch.empty((B, Hq, Q, d), dtype=torch.float32, device=q.device)
-        elif out.dtype != torch.float32 or out.shape != q.shape or not out.is_contiguous() or out.device != self.device:
-            raise ValueError("quashkv_b200: out must be a contiguous fp32 tensor of the queries' shape on their device")
-        need = self.lib.qkv_attention_workspace_bytes(B, Hq, n_kv_heads, Q, kv_len, d)
-        if self.ws is None or self.ws.numel() < need:
-            self.ws = torch.empty((max(need + need // 4, 1 << 16),), dtype=torch.uint8, device=q.device)
-        cache = TiledCache(records.data_ptr(), capacity, None, None, 0, 0)
-        rc = self.fn(qc.data_ptr(), _DT[qc.dtype], cache, B, Hq, n_kv_heads, Q, kv_len, d, 3, 3, *self.ptrs,
-                     self.qjl_scale, scale, int(causal), out.data_ptr(), self.ws.data_ptr(), self.ws.numel(),
-                     torch.cuda.current_stream(q.device).cuda_stream if stream is None else stream)
-        if rc:
-            _lib.check(rc, "attention_tiled")
-        return out
-
-
-@_attention_tiled.register_fake
+@torch.library.register_fake("quashkv_b200::attention_tiled")
 def _(q, records, capacity, kv_len, n_kv_heads, block_table, seq_lens, block_size, Pi, key_centroids,
       val_centroids, S, qjl_scale, scale, causal):
     return q.new_empty(q.shape, dtype=torch.float32)
 
 
-@torch.library.custom_op("quashkv_b200::index_scan_topk", mutates_args=(), device_types="cuda")
-def _index_scan_topk(queries: torch.Tensor, db_codes: torch.Tensor, db_signs: torch.Tensor,
-                     db_norms: torch.Tensor, n_vectors: int, bits: int, Pi: torch.Tensor,
-                     centroids: torch.Tensor, S: torch.Tensor, qjl_scale: float, k: int,
-                     id_base: int) -> tuple[torch.Tensor, torch.Tensor]:
-    qf = _f32(queries)
-    M, d = qf.shape
-    scores = torch.empty((M, k), dtype=torch.float32, device=qf.device)
-    ids = torch.empty((M, k), dtype=torch.int64, device=qf.device)
-    L = _lib.lib()
-    ws_bytes = L.qkv_index_workspace_bytes(n_vectors, M, d, k)
-    ws = torch.empty((max(ws_bytes, 16),), dtype=torch.uint8, device=qf.device)
-    _same_device(qf.device, qf, db_codes, db_signs, db_norms)
-    A = _Keep(qf.device)
-    with torch.cuda.device(qf.device):
-        _lib.check(L.qkv_index_scan_topk(
-            _p(qf), M, d, _p(db_codes), _p(db_signs), _p(db_norms), n_vectors, bits, A.f32(Pi),
-            A.f32(centroids), A.f32(S), float(qjl_scale), k, id_base, _p(scores), _p(ids),
-            _p(ws), ws_bytes, _stream(qf)), "index_scan_topk")
-    return scores, ids
-
-
-@_index_scan_topk.register_fake
+@torch.library.register_fake("quashkv_b200::index_scan_topk")
 def _(queries, db_codes, db_signs, db_norms, n_vectors, bits, Pi, centroids, S, qjl_scale, k, id_base):
     M = queries.shape[0]
     return queries.new_empty((M, k), dtype=torch.float32), queries.new_empty((M, k), dtype=torch.int64)
@@ -754,6 +398,21 @@ def _(scores, ids, k):
     return scores.new_empty((M, k), dtype=torch.float32), ids.new_empty((M, k), dtype=torch.int64)
 
 
+append_kv = _NATIVE.append_kv.default
+append_records = _NATIVE.append_records.default
+compress_ip_into = _NATIVE.compress_ip_into.default
+attention = _NATIVE.attention.default
+attention_paged = _NATIVE.attention_paged.default
+attention_tiled = _attention_tiled = _NATIVE.attention_tiled.default
+attention_tiled_out = _NATIVE.attention_tiled_out.default
+index_scan_topk = _NATIVE.index_scan_topk.default
+_compress_mse = _NATIVE.compress_mse.default
+_compress_ip = _NATIVE.compress_ip.default
+_compress_mixed = _NATIVE.compress_mixed.default
+_decompress = _NATIVE.decompress.default
+_decompress_mixed = _NATIVE.decompress_mixed.default
+
+
 # ---------------------------------------------------------------------------------------------
 # public wrappers
 # ---------------------------------------------------------------------------------------------
@@ -763,6 +422,8 @@ def _need_cuda(t: torch.Tensor, what: str) -> None:
         raise RuntimeError(
             f"quashkv_b200.{what}: expected a CUDA tensor, got device '{t.device}'. The hot path runs "
             "only as sm_100a kernels; there is no CPU implementation.")
+    if not _lib.HOST_READY:
+        _lib.load_host()
 
 
 def pack(codes, bits):
@@ -836,15 +497,9 @@ def decompress_mixed(codes, norms, Pi, is_outlier, cents_out, bits_out, cents_re
                              codes.shape[-1] if d is None else d)
 
 
-append_kv = _append_kv
-compress_ip_into = _compress_ip_into
-attention = _attention
-attention_paged = _attention_paged
 scatter_rows = _scatter_rows
 tile_rows = _tile_rows
 untile_rows = _untile_rows
-attention_tiled = _attention_tiled
-index_scan_topk = _index_scan_topk
 index_scores = _index_scores
 topk_merge = _topk_merge
 INDEX_MAX_K = _lib.INDEX_MAX_K
