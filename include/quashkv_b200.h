@@ -245,6 +245,41 @@ int qkv_attention_paged(const void* q, int q_dtype, qkv_paged_cache_t pool,
 int qkv_scatter_rows(const void* src, void* dst, const int64_t* slots, int64_t n_rows, int row_bytes,
                      void* stream);
 
+/* ---- append: new keys and values straight into a cache ------------------------------------------------
+ * The compression of qkv_compress_ip (keys) and qkv_compress_mse (values) with the result filed where the
+ * cache keeps it.  Stands where the reference compresses a block and appends it to its list
+ * (engine.py:145-172).
+ *   keys, values  (B, H, tokens, d) contiguous, each with its own dtype
+ *   destination   tile records (records != NULL; d = 128, mse_bits = 2, val_bits = 3) or the five
+ *                 row-major planes of qkv_cache_t / qkv_paged_cache_t;
+ *                 contiguous (block_table == NULL): token t of segment b * H + h goes to row
+ *                 (b * H + h) * capacity + offset + t;
+ *                 paged: to position start_lens[b] + t of the pages block_table[b][..], rows of
+ *                 (block * H + h) * block_size + position % block_size; a position outside the table is
+ *                 dropped.
+ *   workspace     qkv_append_workspace_bytes(...) bytes, 256-byte aligned (0 for small appends: they are
+ *                 one launch that writes the cache directly). */
+typedef struct {
+  uint8_t* records;
+  uint8_t* k_codes;
+  uint8_t* k_signs;
+  float* k_norms;
+  uint8_t* v_codes;
+  float* v_norms;
+  int64_t capacity;
+  int64_t offset;
+  const int32_t* block_table;
+  const int32_t* start_lens;
+  int max_blocks;
+  int block_size;
+} qkv_kv_dest_t;
+
+size_t qkv_append_workspace_bytes(int B, int H, int64_t tokens, int d, int mse_bits, int val_bits, int tiled, int paged);
+int qkv_append_kv(const void* keys, int k_dtype, const void* values, int v_dtype, int B, int H, int64_t tokens, int d,
+                  const float* Pi, const float* k_boundaries, const float* k_centroids, const float* S, int mse_bits,
+                  const float* v_boundaries, int val_bits, qkv_kv_dest_t dest,
+                  void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- tile records: the cache layout of the fast decode path -----------------------------------------
  * For head_dim 128 with 3-bit keys (2-bit codes + sign bit) and 3-bit values the cache can be kept as
  * RECORDS of 16 consecutive tokens of one (batch, kv head): QKV_TILE_BYTES = 16 * 104 bytes, the same

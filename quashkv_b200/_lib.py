@@ -42,6 +42,13 @@ class TiledCache(C.Structure):
                 ("max_blocks", _i), ("block_size", _i)]
 
 
+class KvDest(C.Structure):
+    """qkv_kv_dest_t: where an append puts the new tokens."""
+    _fields_ = [("records", _vp), ("k_codes", _vp), ("k_signs", _vp), ("k_norms", _vp), ("v_codes", _vp),
+                ("v_norms", _vp), ("capacity", _i64), ("offset", _i64), ("block_table", _vp), ("start_lens", _vp),
+                ("max_blocks", _i), ("block_size", _i)]
+
+
 TILE_TOKENS, TILE_BYTES = 16, 1664
 
 # symbol -> (restype, argtypes); every symbol include/quashkv_b200.h declares is listed here
@@ -69,6 +76,8 @@ SIGNATURES = {
     "qkv_untile_rows": (_i, [_vp, Rows, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     "qkv_attention_tiled": (_i, [_vp, _i, TiledCache, _i, _i, _i, _i, _i64, _i, _i, _i, _vp, _vp, _vp, _vp, _f, _f,
                                  _i, _vp, _vp, _sz, _vp]),
+    "qkv_append_workspace_bytes": (_sz, [_i, _i, _i64, _i, _i, _i, _i, _i]),
+    "qkv_append_kv": (_i, [_vp, _i, _vp, _i, _i, _i, _i64, _i, _vp, _vp, _vp, _vp, _i, _vp, _i, KvDest, _vp, _sz, _vp]),
     "qkv_scatter_rows": (_i, [_vp, _vp, _vp, _i64, _i, _vp]),
     "qkv_index_workspace_bytes": (_sz, [_i64, _i, _i, _i]),
     "qkv_index_scan_topk": (_i, [_vp, _i, _i, _vp, _vp, _vp, _i64, _i, _vp, _vp, _vp, _f, _i, _i64, _vp, _vp,
@@ -91,7 +100,12 @@ def load_host(required: bool = True) -> None:
     global HOST_READY
     if HOST_READY or (not required and not (os.path.exists(HOST_PATH) and os.path.exists(_path()))):
         return
-    lib()
+    try:
+        lib()
+    except AttributeError:       # a library older than this file: the build that replaces it imports the package too
+        if required:
+            raise
+        return
     if not os.path.exists(HOST_PATH):
         raise RuntimeError(
             f"quashkv_b200: {HOST_PATH} not found. Build it with `python -m quashkv_b200._build`; "

@@ -26,7 +26,7 @@ using OptTensor = std::optional<Tensor>;
 #define QKV_FOR_EACH_ENTRY(X)                                                                                     \
   X(qkv_strerror) X(qkv_compress_mse) X(qkv_compress_ip) X(qkv_compress_mixed) X(qkv_mixed_row_bytes)             \
   X(qkv_decompress) X(qkv_decompress_mixed) X(qkv_attention_workspace_bytes) X(qkv_attention)                     \
-  X(qkv_attention_paged) X(qkv_attention_tiled) X(qkv_tile_rows) X(qkv_index_workspace_bytes) X(qkv_index_scan_topk)
+  X(qkv_attention_paged) X(qkv_attention_tiled) X(qkv_append_workspace_bytes) X(qkv_append_kv) X(qkv_index_workspace_bytes) X(qkv_index_scan_topk)
 
 struct Api {
 #define QKV_MEMBER(name) decltype(&::name) name = nullptr;
@@ -163,55 +163,76 @@ std::tuple<Tensor, Tensor> compress_mixed(const Tensor& x_in, const Tensor& Pi_i
 
 // ---- appends into a cache -----------------------------------------------------------------------------------------
 
-struct KvPlanes { uint8_t* k_codes; uint8_t* k_signs; float* k_norms; uint8_t* v_codes; float* v_norms; };
+struct AppendConsts { Tensor Pi, kb, kc, S, vb; };
 
-void compress_kv(const Tensor& keys, const Tensor& values, const Tensor& Pi, const Tensor& kb, const Tensor& kc,
-                 const Tensor& S, int64_t mse_bits, const Tensor& vb, int64_t val_bits, const KvPlanes& p,
-                 qkv_rows_t rows, void* stream) {
-  const int64_t d = keys.size(-1), n = d > 0 ? keys.numel() / d : 0;
-  check(api.qkv_compress_ip(keys.const_data_ptr(), dtype_code(keys), d, n, d, fp(Pi), fp(kb), fp(kc), mse_bits, fp(S),
-                            p.k_codes, p.k_signs, 1, p.k_norms, rows, stream), "append keys");
-  check(api.qkv_compress_mse(values.const_data_ptr(), dtype_code(values), d, n, d, fp(Pi), fp(vb), val_bits, p.v_codes, 1,
-                             p.v_norms, rows, stream), "append values");
+// (B, H, T, d) keys and values into the destination: one C call.
+void run_append(const Tensor& keys, const Tensor& values, const AppendConsts& c, int64_t mse_bits, int64_t val_bits,
+                const qkv_kv_dest_t& dest, void* stream) {
+  TORCH_CHECK_VALUE(keys.dim() == 4 && keys.sizes() == values.sizes(), "quashkv_b200: keys and values of shape (B, H, S, d)");
+  const at::Device dev = keys.device();
+  const int64_t B = keys.size(0), H = keys.size(1), T = keys.size(2), d = keys.size(3);
+  const int64_t need = api.qkv_append_workspace_bytes(B, H, T, d, mse_bits, val_bits, dest.records != nullptr,
+                                                      dest.block_table != nullptr);
+  const Tensor ws = need > 0 ? empty({need}, at::kByte, dev) : Tensor();
+  const Tensor Pi = f32(c.Pi, dev), kb = f32(c.kb, dev), kc = f32(c.kc, dev), S = f32(c.S, dev), vb = f32(c.vb, dev);
+  check(api.qkv_append_kv(keys.const_data_ptr(), dtype_code(keys), values.const_data_ptr(), dtype_code(values), B, H, T, d,
+                          fp(Pi), fp(kb), fp(kc), fp(S), mse_bits, fp(vb), val_bits, dest,
+                          need > 0 ? ws.data_ptr() : nullptr, need, stream), "append");
 }
 
-// (B, H, S, d) keys and values into row-major planes [B*H, capacity, ...] at rows offset .. offset + S of every segment.
-void append_kv(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi_in, const Tensor& kb_in,
-               const Tensor& kc_in, const Tensor& S_in, int64_t mse_bits, const Tensor& vb_in, int64_t val_bits,
-               Tensor k_codes, Tensor k_signs, Tensor k_norms, Tensor v_codes, Tensor v_norms, int64_t offset) {
+// Row-major planes [B*H, capacity, ...], rows offset .. offset + S of every segment.
+void append_kv(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi, const Tensor& kb, const Tensor& kc,
+               const Tensor& S, int64_t mse_bits, const Tensor& vb, int64_t val_bits, Tensor k_codes, Tensor k_signs,
+               Tensor k_norms, Tensor v_codes, Tensor v_norms, int64_t offset) {
   const Tensor keys = data(keys_in), values = data(values_in);
   const at::Device dev = keys.device();
   Call call(dev);
   same_device(dev, {&values, &k_codes, &k_signs, &k_norms, &v_codes, &v_norms});
-  const Tensor Pi = f32(Pi_in, dev), kb = f32(kb_in, dev), kc = f32(kc_in, dev), S = f32(S_in, dev), vb = f32(vb_in, dev);
-  compress_kv(keys, values, Pi, kb, kc, S, mse_bits, vb, val_bits,
-              {bpm(k_codes), bpm(k_signs), fpm(k_norms), bpm(v_codes), fpm(v_norms)},
-              {keys.size(-2), k_norms.size(-1), offset}, call.stream);
+  qkv_kv_dest_t dest{};
+  dest.k_codes = bpm(k_codes); dest.k_signs = bpm(k_signs); dest.k_norms = fpm(k_norms);
+  dest.v_codes = bpm(v_codes); dest.v_norms = fpm(v_norms);
+  dest.capacity = k_norms.size(-1); dest.offset = offset;
+  run_append(keys, values, {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
 }
 
-// The same into tile records [B*H, capacity / 16, 1664] at tokens offset .. offset + S (slots == nullptr) or at the
-// given token slots: the packed rows go through a staging area, an integer kernel files every token.
-void append_records(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi_in, const Tensor& kb_in,
-                    const Tensor& kc_in, const Tensor& S_in, int64_t mse_bits, const Tensor& vb_in, int64_t val_bits,
-                    Tensor records, int64_t capacity, int64_t offset, const OptTensor& slots) {
+// Tile records [B*H, capacity / 16, 1664], tokens offset .. offset + S of every segment.
+void append_records(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi, const Tensor& kb, const Tensor& kc,
+                    const Tensor& S, int64_t mse_bits, const Tensor& vb, int64_t val_bits, Tensor records,
+                    int64_t capacity, int64_t offset) {
   const Tensor keys = data(keys_in), values = data(values_in);
   const at::Device dev = keys.device();
   Call call(dev);
-  same_device(dev, {&values, &records, slots ? &*slots : nullptr});
-  const Tensor Pi = f32(Pi_in, dev), kb = f32(kb_in, dev), kc = f32(kc_in, dev), S = f32(S_in, dev), vb = f32(vb_in, dev);
-  const int64_t d = keys.size(-1), n = keys.numel() / d, s_new = keys.size(-2);
-  if (n == 0) return;
-  const auto up = [](int64_t b) { return (b + 255) / 256 * 256; };
-  const int64_t pk = up(n * row_bytes(d, mse_bits)), ps = up(n * row_bytes(d, 1)), pv = up(n * row_bytes(d, val_bits));
-  const int64_t pn = up(4 * n);
-  const Tensor stage = empty({pk + ps + pv + 2 * pn}, at::kByte, dev);
-  uint8_t* base = bpm(stage);
-  const KvPlanes p{base, base + pk, reinterpret_cast<float*>(base + pk + ps + pv), base + pk + ps,
-                   reinterpret_cast<float*>(base + pk + ps + pv + pn)};
-  compress_kv(keys, values, Pi, kb, kc, S, mse_bits, vb, val_bits, p, dense(n), call.stream);
-  check(api.qkv_tile_rows(p.k_codes, p.k_signs, p.k_norms, p.v_codes, p.v_norms, n, bpm(records),
-                          {s_new > 1 ? s_new : 1, capacity, offset},
-                          slots ? static_cast<const int64_t*>(slots->const_data_ptr()) : nullptr, call.stream), "tile_rows");
+  same_device(dev, {&values, &records});
+  qkv_kv_dest_t dest{};
+  dest.records = bpm(records);
+  dest.capacity = capacity; dest.offset = offset;
+  run_append(keys, values, {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
+}
+
+// A pool of pages: planes = {records} or the five planes, positions start_lens[b] .. of the pages in block_table.
+void append_paged(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi, const Tensor& kb, const Tensor& kc,
+                  const Tensor& S, int64_t mse_bits, const Tensor& vb, int64_t val_bits, at::TensorList planes,
+                  const Tensor& table_in, const Tensor& lens_in, int64_t block_size) {
+  const Tensor keys = data(keys_in), values = data(values_in);
+  const at::Device dev = keys.device();
+  Call call(dev);
+  for (const Tensor& p : planes) same_device(dev, {&p});
+  same_device(dev, {&values, &table_in, &lens_in});
+  const auto int32 = [](const Tensor& t) { return t.scalar_type() == at::kInt ? t.contiguous() : t.to(at::kInt).contiguous(); };
+  const Tensor table = int32(table_in), lens = int32(lens_in);
+  qkv_kv_dest_t dest{};
+  if (planes.size() == 1) {
+    dest.records = bpm(planes[0]);
+  } else {
+    TORCH_CHECK_VALUE(planes.size() == 5, "quashkv_b200: a pool has one plane of records or five row-major planes");
+    dest.k_codes = bpm(planes[0]); dest.k_signs = bpm(planes[1]); dest.k_norms = fpm(planes[2]);
+    dest.v_codes = bpm(planes[3]); dest.v_norms = fpm(planes[4]);
+  }
+  dest.block_table = static_cast<const int32_t*>(table.const_data_ptr());
+  dest.start_lens = static_cast<const int32_t*>(lens.const_data_ptr());
+  dest.max_blocks = static_cast<int>(table.size(1));
+  dest.block_size = static_cast<int>(block_size);
+  run_append(keys, values, {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
 }
 
 // ---- decompress ---------------------------------------------------------------------------------------------------
@@ -228,6 +249,17 @@ Tensor decompress(const Tensor& codes, const OptTensor& signs, const Tensor& nor
                            n_vec, d, fp(Pi), fp(cents), bits, S_in ? fp(S) : nullptr, static_cast<float>(qjl_scale),
                            out.data_ptr(), out_code(out_dtype), d, call.stream), "decompress");
   return out;
+}
+
+// Dense planes: codes (..., d) or (..., packed bytes), signs of the same leading shape, norms (...).
+Tensor decompress_dense(const Tensor& codes_in, const OptTensor& signs_in, const Tensor& norms_in, const Tensor& Pi,
+                        const Tensor& cents, int64_t bits, const OptTensor& S, double qjl_scale, bool packed, int64_t d,
+                        at::ScalarType out_dtype) {
+  const Tensor codes = codes_in.contiguous(), norms = f32(norms_in, norms_in.device());
+  const OptTensor signs = signs_in ? OptTensor(signs_in->contiguous()) : OptTensor();
+  const int64_t width = codes.size(-1), n = width > 0 ? codes.numel() / width : 0;
+  return decompress(codes, signs, norms, Pi, cents, bits, S, qjl_scale, packed, d, n > 1 ? n : 1, 0, 0, n, out_dtype)
+      .view(lead_shape(codes, d));
 }
 
 Tensor decompress_mixed(const Tensor& codes_in, const Tensor& norms_in, const Tensor& Pi_in, const Tensor& mask_in,
@@ -371,7 +403,7 @@ extern "C" int quashkv_host_bind(const char* path) {
 }
 
 #define QKV_FOR_EACH_OP(X)                                                                                          \
-  X(compress_mse) X(compress_ip) X(compress_ip_into) X(compress_mixed) X(append_kv) X(append_records) X(decompress) \
+  X(compress_mse) X(compress_ip) X(compress_ip_into) X(compress_mixed) X(append_kv) X(append_records) X(append_paged) X(decompress) X(decompress_dense) \
   X(decompress_mixed) X(attention) X(attention_paged) X(attention_tiled) X(attention_tiled_out) X(index_scan_topk)
 
 TORCH_LIBRARY_IMPL(quashkv_b200, CUDA, m) {

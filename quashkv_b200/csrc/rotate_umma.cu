@@ -23,6 +23,8 @@
 //
 // Every wait on the tensor core is bounded; if one runs out the CTA stops using the tensor core,
 // counts the event and derives its remaining tiles with the fp32 chain alone (slow, still exact).
+#include <stdlib.h>
+
 #include <type_traits>
 
 #include "rotate_exact.cuh"
@@ -597,10 +599,10 @@ bool compress_umma_ok(const CompressArgs& a) {
   if (a.mode == MODE_MIXED) {   // bf16 input, the common width pairs; row of 4-byte words (36 B at 32x3 + 96x2)
     const bool pair = (a.bits0 == 3 && a.bits1 == 2) || (a.bits0 == 4 && a.bits1 == 3) || (a.bits0 == 4 && a.bits1 == 2);
     if (!pair || a.x_dtype != QKV_BF16) return false;
-    return a.d == kRD && a.packed && a.n_vec >= 1024 && a.n_vec < (int64_t(1) << 31) && (a.x_pitch & 7) == 0 &&
+    return a.d == kRD && a.packed && a.n_vec >= kTensorCoreVectors && a.n_vec < (int64_t(1) << 31) && (a.x_pitch & 7) == 0 &&
            ((reinterpret_cast<uintptr_t>(a.x) & 15u) | (reinterpret_cast<uintptr_t>(a.codes) & 3u)) == 0;
   }
-  return a.d == kRD && a.packed && a.n_vec >= 1024 && a.n_vec < (int64_t(1) << 31) &&
+  return a.d == kRD && a.packed && a.n_vec >= kTensorCoreVectors && a.n_vec < (int64_t(1) << 31) &&
          (a.x_pitch & 7) == 0 && (al & 15u) == 0;
 }
 

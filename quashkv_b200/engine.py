@@ -122,11 +122,10 @@ class QuashKVEngine:
         p = self._planes
         consts = (Pi, k_bounds, k_cents, Sgn, kq.mse_bits, v_bounds, self.value_bits)
         if self._tiled:
-            # packed rows go through a staging area, an exact integer kernel files every token into its record
             records = p["records"]
             if (b, H) != self._shape or seg0:
                 records = records[seg0:seg0 + b * H]
-            ops.append_records(keys, values, *consts, records, self._capacity, offset, None)
+            ops.append_records(keys, values, *consts, records, self._capacity, offset)
             return
         planes = (p["k_codes"], p["k_signs"], p["k_norms"], p["v_codes"], p["v_norms"])
         if (b, H) != self._shape or seg0:

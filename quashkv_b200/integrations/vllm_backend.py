@@ -237,15 +237,12 @@ class QuashKVPagedCache:
                              f"{self.head_size})")
         if T == 0:
             return
-        bs = self.block_size
-        slots = np.empty((n, H, T), dtype=np.int64)
-        for i, s in enumerate(seq_ids):
+        starts = np.asarray([self._lens.get(s, 0) for s in seq_ids], dtype=np.int32)
+        for s in seq_ids:
             self._grow(s, T)
-            pos = self._lens.get(s, 0) + np.arange(T)
-            blk = np.asarray(self._blocks[s], dtype=np.int64)[pos // bs]
-            slots[i] = (blk[None, :] * H + np.arange(H)[:, None]) * bs + (pos % bs)[None, :]
             self._lens[s] = self._lens.get(s, 0) + T
-        self._store(keys, values, torch.from_numpy(slots.reshape(-1)).to(self.device))
+        table, _, _ = self.block_table(seq_ids)
+        self._store(keys, values, table, torch.from_numpy(starts).to(self.device))
 
     def append_with_tables(self, keys: torch.Tensor, values: torch.Tensor, block_table: torch.Tensor,
                            start_lens: torch.Tensor) -> None:
@@ -262,32 +259,16 @@ class QuashKVPagedCache:
                              "a block table and start lengths for n_seq sequences")
         if T == 0:
             return
-        bs = self.block_size
-        dev = keys.device
-        pos = start_lens.to(torch.int64).reshape(n, 1) + torch.arange(T, device=dev, dtype=torch.int64).reshape(1, T)
-        blk = torch.gather(block_table.to(torch.int64), 1, torch.div(pos, bs, rounding_mode="floor"))       # (n, T)
-        heads = torch.arange(H, device=dev, dtype=torch.int64).reshape(1, H, 1)
-        slots = (blk.reshape(n, 1, T) * H + heads) * bs + (pos % bs).reshape(n, 1, T)
-        self._store(keys, values, slots.reshape(-1).contiguous())
+        self._store(keys, values, block_table, start_lens)
 
-    def _store(self, keys: torch.Tensor, values: torch.Tensor, slots_d: torch.Tensor) -> None:
+    def _store(self, keys: torch.Tensor, values: torch.Tensor, table: torch.Tensor, starts: torch.Tensor) -> None:
         """Compress (n_seq, heads, T, d) keys and values and file every token at its slot
-        ((block * heads + head) * block_size + offset)."""
-        n, H, T, D = keys.shape
+        ((block * heads + head) * block_size + offset), which the kernel computes from the table."""
         kq, vq = self.engine.key_quantizer, self.engine.value_quantizer
         Pi, k_bounds, k_cents, Sgn = kq._on(keys.device)
         _, v_bounds, _ = vq._on(keys.device)
-        codes, signs, k_norms = ops.compress_ip(keys, Pi, k_bounds, k_cents, Sgn, kq.mse_bits, packed=True)
-        v_codes, v_norms = ops.compress_mse(values, Pi, v_bounds, self.config.value_bits, packed=True)
-        p = self.planes
-        if self.tiled:
-            flat = lambda t: t.reshape(n * H * T, -1).contiguous()      # noqa: E731
-            ops.tile_rows(flat(codes), flat(signs), k_norms.reshape(-1).contiguous(), flat(v_codes),
-                          v_norms.reshape(-1).contiguous(), p["records"], 1, 0, 0, slots_d)
-            return
-        for src, name in ((codes, "k_codes"), (signs, "k_signs"), (k_norms, "k_norms"),
-                          (v_codes, "v_codes"), (v_norms, "v_norms")):
-            ops.scatter_rows(src.contiguous(), p[name], slots_d)
+        ops.append_paged(keys, values, Pi, k_bounds, k_cents, Sgn, kq.mse_bits, v_bounds, self.config.value_bits,
+                         list(self.planes.values()), table, starts, self.block_size)
 
     def rows_of(self, seq_id) -> dict:
         """The stored tokens of one sequence as the five packed planes ``[num_kv_heads, tokens, ...]`` in the

@@ -103,10 +103,13 @@ for _schema in (
         "int bits_reg, bool packed, int n_out) -> (Tensor, Tensor)",
         f"append_kv({_APPEND}, Tensor(a!) k_codes, Tensor(b!) k_signs, Tensor(c!) k_norms, Tensor(d!) v_codes, "
         "Tensor(e!) v_norms, int offset) -> ()",
-        f"append_records({_APPEND}, Tensor(a!) records, int capacity, int offset, Tensor? slots) -> ()",
+        f"append_records({_APPEND}, Tensor(a!) records, int capacity, int offset) -> ()",
+        f"append_paged({_APPEND}, Tensor(a!)[] planes, Tensor block_table, Tensor start_lens, int block_size) -> ()",
         "decompress(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, int bits, Tensor? S, "
         "float qjl_scale, bool packed, int d, int seg_len, int seg_stride, int seg_off, int n_vec, "
         "ScalarType out_dtype) -> Tensor",
+        "decompress_dense(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, int bits, Tensor? S, "
+        "float qjl_scale, bool packed, int d, ScalarType out_dtype) -> Tensor",
         "decompress_mixed(Tensor codes, Tensor norms, Tensor Pi, Tensor is_outlier, Tensor cents_out, int bits_out, "
         "Tensor cents_reg, int bits_reg, bool packed, int d) -> Tensor",
         "attention(Tensor q, Tensor k_codes, Tensor k_signs, Tensor k_norms, Tensor v_codes, Tensor v_norms, "
@@ -229,6 +232,11 @@ def _(x, Pi, is_outlier, bounds_out, cents_out, bits_out, bounds_reg, cents_reg,
 def _(codes, signs, norms, Pi, centroids, bits, S, qjl_scale, packed, d, seg_len, seg_stride, seg_off,
       n_vec, out_dtype):
     return codes.new_empty((n_vec, d), dtype=out_dtype)
+
+
+@torch.library.register_fake("quashkv_b200::decompress_dense")
+def _(codes, signs, norms, Pi, centroids, bits, S, qjl_scale, packed, d, out_dtype):
+    return codes.new_empty((*codes.shape[:-1], d), dtype=out_dtype)
 
 
 @torch.library.register_fake("quashkv_b200::decompress_mixed")
@@ -400,6 +408,7 @@ def _(scores, ids, k):
 
 append_kv = _NATIVE.append_kv.default
 append_records = _NATIVE.append_records.default
+append_paged = _NATIVE.append_paged.default
 compress_ip_into = _NATIVE.compress_ip_into.default
 attention = _NATIVE.attention.default
 attention_paged = _NATIVE.attention_paged.default
@@ -410,6 +419,7 @@ _compress_mse = _NATIVE.compress_mse.default
 _compress_ip = _NATIVE.compress_ip.default
 _compress_mixed = _NATIVE.compress_mixed.default
 _decompress = _NATIVE.decompress.default
+_decompress_dense = _NATIVE.decompress_dense.default
 _decompress_mixed = _NATIVE.decompress_mixed.default
 
 
@@ -471,15 +481,8 @@ def decompress(codes, norms, Pi, centroids, bits, *, signs=None, S=None, qjl_sca
                d=None, out_dtype=torch.float32):
     """Dense planes: codes (..., d) or (..., packed bytes), norms (...)."""
     _need_cuda(codes, "decompress")
-    if d is None:
-        d = codes.shape[-1]
-    lead = codes.shape[:-1]
-    flat = codes.reshape(-1, codes.shape[-1]).contiguous()
-    sflat = None if signs is None else signs.reshape(-1, signs.shape[-1]).contiguous()
-    n = flat.shape[0]
-    out = _decompress(flat, sflat, _f32(norms).reshape(-1), Pi, centroids, bits, S, qjl_scale, packed, d,
-                      max(n, 1), 0, 0, n, out_dtype)
-    return out.reshape(*lead, d)
+    return _decompress_dense(codes, signs, norms, Pi, centroids, bits, S, qjl_scale, packed,
+                             codes.shape[-1] if d is None else d, out_dtype)
 
 
 def decompress_rows(codes, norms, Pi, centroids, bits, d, n_seg, seg_len, seg_stride, seg_off, *,
