@@ -21,6 +21,10 @@
 // together (a flag out of the tile barrier), and the products of a tile are issued one at a time between the
 // phases of the loop, because the issuing thread is held for about as long as its MMAs execute.
 //
+// One byte per coordinate (the unpacked form of the quantizer classes) leaves through the same epilogue: the fp32
+// kernels that took it before ran at a fifth of the FMA rate, most of it spent on scattering single bytes.  204795
+// vectors of bf16 with signs 509 -> 102 us, 65537 of fp32 at 4 bits 125 -> 71 us.
+//
 // Every wait on the tensor core is bounded; if one runs out the CTA stops using the tensor core,
 // counts the event and derives its remaining tiles with the fp32 chain alone (slow, still exact).
 #include <stdlib.h>
@@ -230,6 +234,14 @@ __global__ void __launch_bounds__(kUThreads, 1) compress_umma_kernel(CompressArg
         for (int b = 0; b < (1 << bits_c) - 1; ++b) code += z > bnd_s[cls][b] ? 1u : 0u;
         const int64_t row = map_row(a.rows, n);
         const uint32_t diff = code ^ old_code;
+        if (!MIXED && !a.packed) {                 // one byte per coordinate
+          if (diff) a.codes[row * kRD + col] = static_cast<uint8_t>(code);
+          if (IP) {
+            const uint32_t sign = ((z - cent_s[code]) * sgn_s[col] >= 0.f) ? 1u : 0u;
+            if (sign != old_sign) a.signs[row * kRD + col] = static_cast<uint8_t>(sign);
+          }
+          continue;
+        }
         if (diff) {
           const int bit = cls ? n_out * BITS + (col - n_out) * BITS1 : col * BITS, w = bit >> 5, sh = bit & 31;
           atomicXor(out_codes + row * row_words + w, diff << sh);
@@ -474,7 +486,33 @@ __global__ void __launch_bounds__(kUThreads, 1) compress_umma_kernel(CompressArg
       }
       fmask = 0xFFFFFFFFu;
     }
-    if (live) {
+    // unflagged coordinates: sign = residual >= 0 exclusive-or S < 0 (a zero residual is always flagged)
+    const uint32_t sign_word = IP ? ((~(__brev(R) ^ smask) & ~fmask) | fval) : 0u;
+    if (!MIXED && !a.packed) {
+      // One byte per coordinate: a thread holds 32 neighbouring bytes of a row, a whole sector, and four codes leave
+      // the packed words with one extraction and two spreads.
+      if (live) {
+        uint4* dst = reinterpret_cast<uint4*>(a.codes + row * kRD + col0);
+        uint4* sdst = IP ? reinterpret_cast<uint4*>(a.signs + row * kRD + col0) : nullptr;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t o[4], so[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int c = 16 * h + 4 * q, bit = BW * c, w = bit >> 5, sh = bit & 31;
+            const uint32_t f = sh ? __funnelshift_r(wb[w], wb[w + 1], sh) : wb[w];
+            constexpr uint32_t m = (1u << BW) - 1u;
+            o[q] = (f & m) | ((f & (m << BW)) << (8 - BW)) | ((f & (m << (2 * BW))) << (16 - 2 * BW)) |
+                   ((f & (m << (3 * BW))) << (24 - 3 * BW));
+            const uint32_t g = sign_word >> c;
+            so[q] = (g & 1u) | ((g & 2u) << 7) | ((g & 4u) << 14) | ((g & 8u) << 21);
+          }
+          dst[h] = make_uint4(o[0], o[1], o[2], o[3]);
+          if (IP) sdst[h] = make_uint4(so[0], so[1], so[2], so[3]);
+        }
+        if (blk == 0) a.norms[row] = nrm;
+      }
+    } else if (live) {
       uint32_t* dst = out_codes + row * row_words + word_off;
       if (!MIXED && BW == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(wb[0], wb[1], wb[2], wb[BW - 1]);
       else if (!MIXED && BW == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(wb[0], wb[1]);
@@ -482,11 +520,7 @@ __global__ void __launch_bounds__(kUThreads, 1) compress_umma_kernel(CompressArg
 #pragma unroll
         for (int w = 0; w < BW; ++w) dst[w] = wb[w];
       }
-      if (IP) {
-        // unflagged coordinates: sign = residual >= 0 exclusive-or S < 0 (a zero residual is always flagged)
-        const uint32_t sw = ~(__brev(R) ^ smask);
-        out_signs[row * (kRD / 32) + blk] = (sw & ~fmask) | fval;
-      }
+      if (IP) out_signs[row * (kRD / 32) + blk] = sign_word;
       if (blk == 0) a.norms[row] = nrm;
     }
     __syncwarp();
@@ -602,7 +636,7 @@ bool compress_umma_ok(const CompressArgs& a) {
     return a.d == kRD && a.packed && a.n_vec >= kTensorCoreVectors && a.n_vec < (int64_t(1) << 31) && (a.x_pitch & 7) == 0 &&
            ((reinterpret_cast<uintptr_t>(a.x) & 15u) | (reinterpret_cast<uintptr_t>(a.codes) & 3u)) == 0;
   }
-  return a.d == kRD && a.packed && a.n_vec >= kTensorCoreVectors && a.n_vec < (int64_t(1) << 31) &&
+  return a.d == kRD && a.n_vec >= kTensorCoreVectors && a.n_vec < (int64_t(1) << 31) &&
          (a.x_pitch & 7) == 0 && (al & 15u) == 0;
 }
 
