@@ -240,33 +240,100 @@ __global__ void topk_merge_kernel(const float* __restrict__ in_s, const int64_t*
             out_s + static_cast<int64_t>(m) * k_out, out_i + static_cast<int64_t>(m) * k_out, lane);
 }
 
-// Long candidate lists (few queries, many slices): one CTA of eight warps per query.  Every warp reduces an
-// eighth of the list to its k best in shared memory, then the first warp merges those 8 k.
-constexpr int kWideWarps = 8;
+// Long candidate lists (few queries, many slices): one CTA of 32 warps per query.  A warp takes its share of the list
+// eight entries per lane at a time into registers, all loads in flight, together with the k best so far (from shared
+// memory), and picks k in rank order with one exchange over the warp each; the first warp then does the same with the
+// warps' lists.  Bound by latency: the kernel before it walked over the list in memory once per result, which took
+// 72 us for 7700 entries and k = 10.
+constexpr int kWideWarps = 32;
+constexpr int kWideNew = 8, kWideOld = QKV_INDEX_MAX_K / 32;
+
+// The k best of s[0 .. n) in rank order to (os, oi), in shared memory; equal (score, id) pairs count once, as in
+// warp_topk.  Entries are read with a stride of 32 from `lane`.
+__device__ __forceinline__ void warp_topk_registers(const float* s, const int64_t* ids, int64_t n, int k, float* os, int64_t* oi,
+                                                    int lane) {
+  int held = 0;                                   // results so far in (os, oi)
+  for (int64_t base = 0; base < n; base += 32 * kWideNew) {
+    float v[kWideNew + kWideOld];
+    int64_t id[kWideNew + kWideOld];
+#pragma unroll
+    for (int e = 0; e < kWideNew; ++e) {
+      const int64_t p = base + lane + 32 * e;
+      v[e] = p < n ? s[p] : -INFINITY;
+      id[e] = p < n ? ids[p] : -1;
+    }
+#pragma unroll
+    for (int e = 0; e < kWideOld; ++e) {
+      const int p = lane + 32 * e;
+      v[kWideNew + e] = p < held ? os[p] : -INFINITY;
+      id[kWideNew + e] = p < held ? oi[p] : -1;
+    }
+    __syncwarp();
+    float prev_s = INFINITY; int64_t prev_i = -1; bool have_prev = false;
+    float best = -INFINITY; int64_t best_i = -1;      // this lane's best entry that ranks after the previous result
+    auto refresh = [&]() {
+      best = -INFINITY; best_i = -1;
+#pragma unroll
+      for (int e = 0; e < kWideNew + kWideOld; ++e) {
+        if (id[e] < 0 || (have_prev && !ranks_before(prev_s, prev_i, v[e], id[e]))) continue;
+        if (best_i < 0 || ranks_before(v[e], id[e], best, best_i)) { best = v[e]; best_i = id[e]; }
+      }
+    };
+    refresh();
+    int r = 0;
+    for (; r < k; ++r) {
+      float w = best; int64_t wi = best_i;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float w2 = __shfl_xor_sync(QKV_FULL_MASK, w, o);
+        const int64_t i2 = __shfl_xor_sync(QKV_FULL_MASK, wi, o);
+        if (i2 >= 0 && (wi < 0 || ranks_before(w2, i2, w, wi))) { w = w2; wi = i2; }
+      }
+      if (wi < 0) break;
+      if (lane == 0) { os[r] = w; oi[r] = wi; }
+      prev_s = w; prev_i = wi; have_prev = true;
+      if (best_i == wi) refresh();
+    }
+    held = r;
+    __syncwarp();
+  }
+  for (int r = held + lane; r < k; r += 32) { os[r] = -INFINITY; oi[r] = -1; }
+  __syncwarp();
+}
+
 __global__ void __launch_bounds__(kWideWarps * 32)
 topk_merge_wide_kernel(const float* __restrict__ in_s, const int64_t* __restrict__ in_i, int M, int64_t n_cand,
                        int k_out, float* __restrict__ out_s, int64_t* __restrict__ out_i,
                        const int* __restrict__ qlist) {
-  __shared__ float part_s[kWideWarps * QKV_INDEX_MAX_K];
-  __shared__ int64_t part_i[kWideWarps * QKV_INDEX_MAX_K];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int mc = blockIdx.x;
   if (mc >= (qlist ? qlist[M] : M)) return;                                 // CTA-uniform
   const int m = qlist ? qlist[mc] : mc;
+  int64_t* part_i = reinterpret_cast<int64_t*>(smem_raw);                   // [warps + 1][k]
+  float* part_s = reinterpret_cast<float*>(part_i + (kWideWarps + 1) * k_out);
   const int64_t chunk = (n_cand + kWideWarps - 1) / kWideWarps;
   const int64_t lo = warp * chunk, hi = lo + chunk < n_cand ? lo + chunk : n_cand;
-  warp_topk(in_s + static_cast<int64_t>(mc) * n_cand + lo, in_i + static_cast<int64_t>(mc) * n_cand + lo,
-            hi > lo ? hi - lo : 0, k_out, part_s + warp * k_out, part_i + warp * k_out, lane);
+  warp_topk_registers(in_s + static_cast<int64_t>(mc) * n_cand + lo, in_i + static_cast<int64_t>(mc) * n_cand + lo,
+                      hi > lo ? hi - lo : 0, k_out, part_s + warp * k_out, part_i + warp * k_out, lane);
   __syncthreads();
-  if (warp == 0)
-    warp_topk(part_s, part_i, kWideWarps * k_out, k_out, out_s + static_cast<int64_t>(m) * k_out,
-              out_i + static_cast<int64_t>(m) * k_out, lane);
+  if (warp == 0) {
+    float* fs = part_s + kWideWarps * k_out;
+    int64_t* fi = part_i + kWideWarps * k_out;
+    warp_topk_registers(part_s, part_i, kWideWarps * k_out, k_out, fs, fi, lane);
+    for (int r = lane; r < k_out; r += 32) {
+      out_s[static_cast<int64_t>(m) * k_out + r] = fs[r];
+      out_i[static_cast<int64_t>(m) * k_out + r] = fi[r];
+    }
+  }
 }
 
 static void launch_topk_merge(const float* in_s, const int64_t* in_i, int M, int64_t n_cand, int k_out,
                               float* out_s, int64_t* out_i, const int* qlist, cudaStream_t st) {
   if (n_cand >= 2048 && k_out <= QKV_INDEX_MAX_K) {
-    topk_merge_wide_kernel<<<M, kWideWarps * 32, 0, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i, qlist);
+    const size_t smem = static_cast<size_t>(kWideWarps + 1) * k_out * 12;
+    if (smem > 49152) cudaFuncSetAttribute(topk_merge_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    topk_merge_wide_kernel<<<M, kWideWarps * 32, smem, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i, qlist);
   } else {
     const int warps = 4;
     topk_merge_kernel<<<(M + warps - 1) / warps, warps * 32, 0, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i,
