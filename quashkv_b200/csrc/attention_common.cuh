@@ -161,45 +161,38 @@ unsigned int bulk_copy_timeouts();        // bounded waits on a record copy that
 // value table, the positive half of a symmetric table) as fp16 pairs for the sign-and-magnitude records,
 // [10] contract flags (bit 0: the value table is not symmetric, bit 1: the key table is not affine in the two
 // bits of its code), [11..13] g0, g1, g2 of the key table written as c(u) = g0 + g1 (u & 1) + g2 (u >> 1).
-// The scale in [1, 2) of a table of n <= 8 values: a CTA-wide call (first 128 threads search four candidates each,
-// everyone passes the barriers), every thread gets the result.  Deterministic: smallest error, then smallest scale.
+// The scale in [1, 2) of a table of n <= 8 values: a CTA-wide call (every thread takes its share of the 512 candidates
+// and passes the barriers), every thread gets the result.  Deterministic: smallest error, then smallest scale.
+// It sits in front of every short call, so it is written for latency: one division per table value and per candidate
+// instead of one per pair, all threads of the CTA at work (before, four candidates on each of 128 threads).
 __device__ inline float best_fp16_scale_cta(const float* __restrict__ cent, int n) {
-  __shared__ float cand_err[4];
-  __shared__ float cand_s[4];
-  __shared__ float chosen;
-  const int tid = threadIdx.x;
-  if (tid < 128) {
-    float c[8];
-    for (int i = 0; i < 8; ++i) c[i] = i < n ? cent[i] : 0.f;
-    float best_err = 1e30f, best_s = 1.f;
-    for (int k = 0; k < 4; ++k) {
-      const float s = 1.f + static_cast<float>(tid + 128 * k) * (1.f / 512.f);
-      float err = 0.f;
+  __shared__ unsigned long long warp_best[32];
+  float c[8], inv[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float v = c[i] * s;
-        if (v != 0.f) err = fmaxf(err, fabsf(__half2float(__float2half_rn(v)) - v) / fabsf(v));
-      }
-      if (err < best_err) { best_err = err; best_s = s; }
-    }
+  for (int i = 0; i < 8; ++i) {
+    c[i] = i < n ? cent[i] : 0.f;
+    inv[i] = c[i] != 0.f ? 1.f / fabsf(c[i]) : 0.f;
+  }
+  unsigned best_err = 0xffffffffu, best_k = 0u;
+  for (int k = threadIdx.x; k < 512; k += blockDim.x) {
+    const float s = 1.f + static_cast<float>(k) * (1.f / 512.f);
+    float err = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float e2 = __shfl_xor_sync(0xffffffffu, best_err, o), s2 = __shfl_xor_sync(0xffffffffu, best_s, o);
-      if (e2 < best_err || (e2 == best_err && s2 < best_s)) { best_err = e2; best_s = s2; }
+    for (int i = 0; i < 8; ++i) {
+      const float v = c[i] * s;
+      err = fmaxf(err, fabsf(__half2float(__float2half_rn(v)) - v) * inv[i]);
     }
-    if ((tid & 31) == 0) { cand_err[tid >> 5] = best_err; cand_s[tid >> 5] = best_s; }
+    const unsigned e = __float_as_uint(err * (1.f / s));         // not negative: ordered as its bits
+    if (e < best_err) { best_err = e; best_k = static_cast<unsigned>(k); }
   }
+  const unsigned w_err = __reduce_min_sync(0xffffffffu, best_err);
+  const unsigned w_k = __reduce_min_sync(0xffffffffu, best_err == w_err ? best_k : 0xffffffffu);
+  if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = (static_cast<unsigned long long>(w_err) << 32) | w_k;
   __syncthreads();
-  if (tid == 0) {
-    float e = 1e30f, s = 1.f;
-    for (int i = 0; i < 4; ++i)
-      if (cand_err[i] < e || (cand_err[i] == e && cand_s[i] < s)) { e = cand_err[i]; s = cand_s[i]; }
-    chosen = s;
-  }
-  __syncthreads();
-  const float r = chosen;
+  unsigned long long best = warp_best[0];
+  for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) best = warp_best[w] < best ? warp_best[w] : best;
   __syncthreads();                          // the scratch may be reused by the next call
-  return r;
+  return 1.f + static_cast<float>(static_cast<unsigned>(best)) * (1.f / 512.f);
 }
 
 __device__ inline void prepare_tables_cta(const float* __restrict__ kcent, const float* __restrict__ vcent,
