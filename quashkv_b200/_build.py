@@ -18,7 +18,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libquashkv_b200.so")
 HOST_PATH = os.path.join(LIB_DIR, "quashkv_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host_ops.cpp")
-SOURCES = ["rotate_quant.cu", "rotate_chain.cu", "rotate_umma.cu", "decompress_umma.cu", "packing.cu", "attention.cu", "attention_mma.cu", "attention_tiled.cu", "tiling.cu", "append.cu", "index_scan.cu", "index_scan_mma.cu", "index_scan_umma.cu"]
+SOURCES = ["rotate_quant.cu", "rotate_chain.cu", "rotate_umma.cu", "decompress_umma.cu", "packing.cu", "attention.cu", "attention_mma.cu", "attention_tiled.cu", "attention_prefill.cu", "tiling.cu", "append.cu", "index_scan.cu", "index_scan_mma.cu", "index_scan_umma.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",

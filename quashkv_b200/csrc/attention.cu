@@ -13,6 +13,7 @@
 //   3. merge_splits: combines the splits of a query row and applies Pi once
 //      (out = (acc / sum) @ Pi), which equals un-rotating every value first because the
 //      rotation is linear.
+// Calls with many query rows go to attention_prefill.cu where that pays, tile records to attention_tiled.cu.
 #include <math.h>
 #include <stdlib.h>
 
@@ -663,10 +664,15 @@ static AttnKernel pick(int wk, int wv) {
 
 using namespace qkv;
 
-extern "C" size_t qkv_attention_workspace_bytes(int B, int Hq, int Hkv, int q_len, int64_t kv_len, int d) {
-  if (B < 1 || Hq < 1 || Hkv < 1 || q_len < 1 || kv_len < 1 || d < 32) return 0;
+static size_t plan_bytes(int B, int Hq, int Hkv, int q_len, int64_t kv_len, int d) {
   const AttnPlan p = make_plan(B, Hq, Hkv, q_len, kv_len, d);
   return p.hdr_bytes + p.qk_bytes + p.part_bytes;
+}
+
+extern "C" size_t qkv_attention_workspace_bytes(int B, int Hq, int Hkv, int q_len, int64_t kv_len, int d) {
+  if (B < 1 || Hq < 1 || Hkv < 1 || q_len < 1 || kv_len < 1 || d < 32) return 0;
+  const size_t plan = plan_bytes(B, Hq, Hkv, q_len, kv_len, d), prefill = qkv::prefill_workspace_bytes(B, Hq, Hkv, q_len, kv_len, d);
+  return plan > prefill ? plan : prefill;
 }
 
 namespace {
@@ -722,6 +728,20 @@ int attention_run(const void* q, int q_dtype, qkv_cache_t cache, const uint8_t* 
   const bool chunks_ok = (paged ? paged->block_size % 16 == 0 : cache.capacity % 4 == 0) &&
       ((reinterpret_cast<uintptr_t>(cache.k_norms) | reinterpret_cast<uintptr_t>(cache.v_norms)) & 15u) == 0;
   const bool use_mma = tiled || (mma_path_ok(d, key_bits, val_bits, Hq / Hkv, q_len) && chunks_ok && !force_generic);
+  AttnArgs a{};
+  a.cache = cache; a.B = B; a.Hq = Hq; a.Hkv = Hkv; a.G = Hq / Hkv; a.q_len = q_len; a.d = d;
+  a.causal = causal; a.kv_len = kv_len; a.qk = qk; a.kcent = key_centroids; a.vcent = val_centroids;
+  a.part = part; a.n_splits = p.n_splits; a.split_len = p.split_len;
+  if (paged) {
+    a.block_table = paged->block_table; a.seq_lens = paged->seq_lens;
+    a.max_blocks = paged->max_blocks; a.block_size = paged->block_size;
+  }
+  a.records = records;
+  a.Pi = Pi;
+  a.out = out;
+  // (planes at d = 128, 3/3 bits keep the mma.sync kernel, whose tables and roundings are its own)
+  if (!force_generic && (tiled || !use_mma) && prefill_ok(a, workspace_bytes))
+    return launch_prefill(a, q, q_dtype, key_bits, val_bits, S, qjl_scale, scale, workspace, st);
   // tile records with up to four query rows per KV head: scores from bit planes, operands built by the rotation
   const bool from_planes = tiled && tiled_scores_from_planes(Hq / Hkv, q_len);
   PlaneImage* planes = from_planes ? reinterpret_cast<PlaneImage*>(ws + p.img_off) : nullptr;
@@ -755,22 +775,11 @@ int attention_run(const void* q, int q_dtype, qkv_cache_t cache, const uint8_t* 
   }
   if (rc) return rc;
 
-  AttnArgs a{};
-  a.cache = cache; a.B = B; a.Hq = Hq; a.Hkv = Hkv; a.G = Hq / Hkv; a.q_len = q_len; a.d = d;
-  a.causal = causal; a.kv_len = kv_len; a.qk = qk; a.kcent = key_centroids; a.vcent = val_centroids;
-  a.part = part; a.n_splits = p.n_splits; a.split_len = p.split_len;
-  if (paged) {
-    a.block_table = paged->block_table; a.seq_lens = paged->seq_lens;
-    a.max_blocks = paged->max_blocks; a.block_size = paged->block_size;
-  }
   if (use_mma) {          // one launch: the last split of every (batch, kv head) merges and un-rotates
     a.tables = tables;
     const int64_t grid_ctas = static_cast<int64_t>(B) * Hkv * (((Hq / Hkv) * q_len + 7) / 8) * p.n_splits;
     a.skew = grid_ctas >= 2 * 4 * kNumSMs ? kSplitSkew : 0.f;
     a.arrivals = reinterpret_cast<unsigned*>(ws + kAttnHeaderBytes);
-    a.Pi = Pi;
-    a.out = out;
-    a.records = records;
     a.planes = planes;
     a.groups = groups;
     return tiled ? launch_attend_tiled(a, st) : launch_attend_mma(a, st);
@@ -843,8 +852,8 @@ extern "C" int qkv_attention_static_scratch(const void* q, int q_dtype, qkv_cach
                                             const float* val_centroids, const float* S, float qjl_scale,
                                             float scale, int causal, float* out, void* stream) {
   if (B < 1 || Hq < 1 || Hkv < 1 || q_len < 1 || kv_len < 1 || d < 32 || d > kMaxD) return QKV_EDIM;
-  const size_t need = qkv_attention_workspace_bytes(B, Hq, Hkv, q_len, kv_len, d);
-  if (need == 0 || need > QKV_ATTENTION_STATIC_SCRATCH_BYTES) return QKV_EWORKSPACE;
+  const size_t need = plan_bytes(B, Hq, Hkv, q_len, kv_len, d);      // (the prefill kernels run when they fit as well)
+  if (need > QKV_ATTENTION_STATIC_SCRATCH_BYTES) return QKV_EWORKSPACE;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return QKV_EARG;
   void* ptr = __atomic_load_n(&g_scratch_addr[dev], __ATOMIC_ACQUIRE);

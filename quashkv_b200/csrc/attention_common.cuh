@@ -151,6 +151,12 @@ int launch_attend_mma(const AttnArgs& a, cudaStream_t st);
 bool tiled_path_ok(int d, int key_bits, int val_bits);
 bool tiled_scores_from_planes(int group, int q_len);      // up to four query rows per KV head (and not switched off)
 int launch_attend_tiled(const AttnArgs& a, cudaStream_t st);
+// Many query rows on tcgen05 (attention_prefill.cu).  From kPrefillRows rows per KV head on it is the faster one.
+constexpr int64_t kPrefillRows = 64;
+bool prefill_ok(const AttnArgs& a, size_t workspace_bytes);
+size_t prefill_workspace_bytes(int B, int Hq, int Hkv, int q_len, int64_t kv_len, int d);      // 0: never taken
+int launch_prefill(const AttnArgs& a, const void* q, int q_dtype, int key_bits, int val_bits, const float* S, float qjl_scale,
+                   float scale, void* workspace, cudaStream_t st);
 unsigned int bulk_copy_timeouts();        // bounded waits on a record copy that ran out (device-wide counter)
 
 // Look-up tables of the tensor-core path, built by one CTA of 128 threads.  For each table the scale

@@ -180,9 +180,9 @@ extern "C" int qkv_decompress_mixed(const uint8_t* codes, int packed, const floa
   return run_decompress(a, static_cast<cudaStream_t>(stream));
 }
 
-namespace qkv { unsigned int index_umma_timeouts(); unsigned int bulk_copy_timeouts(); }
+namespace qkv { unsigned int index_umma_timeouts(); unsigned int bulk_copy_timeouts(); unsigned int prefill_timeouts(); }
 
 extern "C" int64_t qkv_tensor_core_timeouts(void) {
   return static_cast<int64_t>(umma_timeouts()) + static_cast<int64_t>(index_umma_timeouts()) +
-         static_cast<int64_t>(bulk_copy_timeouts());
+         static_cast<int64_t>(bulk_copy_timeouts()) + static_cast<int64_t>(prefill_timeouts());
 }

@@ -4,6 +4,9 @@ import pytest
 import torch
 
 import quashkv_b200 as qk
+from quashkv_b200 import _lib
+from quashkv_b200.integrations.vllm_backend import QuashKVPageConfig, QuashKVPagedCache
+from helpers import rel_l2
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -26,3 +29,58 @@ def test_unpacked_codes_equal_the_packed_ones(n, dtype):
         packed, packed_s, norms_p = q.compress_packed(x)
         assert torch.equal(qk.unpack_bits(packed, bits - 1, 128), codes) and torch.equal(norms, norms_p)
         assert torch.equal(qk.unpack_bits(packed_s, 1, 128), signs)
+
+
+def _outliers(g, shape, dtype):
+    x = torch.randn(shape, generator=g, device=DEV)
+    x[..., ::37] *= 8.0
+    return x.to(dtype)
+
+
+@pytest.mark.parametrize("D,kb,vb", [(128, 3, 3), (64, 3, 3), (64, 2, 4), (128, 4, 2), (128, 2, 4)])
+@pytest.mark.parametrize("n,q_len,G,causal,dtype", [
+    (64, 64, 1, True, torch.bfloat16),            # one token tile, half a row tile
+    (65, 65, 2, True, torch.float32),             # one token into the second tile, one row tile and two rows
+    (127, 33, 4, False, torch.float16),           # a short block of queries over an older cache
+    (321, 130, 2, True, torch.bfloat16),          # rows of two heads in one row tile, a ragged end everywhere
+    (1, 1, 160, False, torch.float32),            # a single token
+    (640, 512, 1, True, torch.bfloat16),          # whole row tiles, heaviest first
+])
+def test_prefill_kernels_match_the_decode_kernels(D, kb, vb, n, q_len, G, causal, dtype, monkeypatch):
+    """The same call through the kernels of long and of short query blocks.  Both hold fp32 (about 5e-7 from 64-bit
+    results) but at d = 128, 3/3 bits, where each rounds queries, tables and weights to fp16 (about 4e-4)."""
+    g = torch.Generator(device=DEV).manual_seed(n + D)
+    eng = qk.QuashKVEngine(D, kb, vb, seed=42, device=DEV, pack_storage=True)
+    eng.append(_outliers(g, (2, 2, n, D), dtype), _outliers(g, (2, 2, n, D), dtype))
+    q = torch.randn(2, 2 * G, q_len, D, generator=g, device=DEV).to(dtype)
+    monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "0")
+    want = eng.attention(q, causal=causal)
+    monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "1")
+    before = _lib.lib().qkv_tensor_core_timeouts()
+    got = eng.attention(q, causal=causal)
+    assert _lib.lib().qkv_tensor_core_timeouts() == before
+    assert rel_l2(got, want) < (1e-3 if (D, kb, vb) == (128, 3, 3) else 5e-6)
+
+
+@pytest.mark.parametrize("D,block", [(128, 16), (128, 48), (64, 16), (64, 20)])
+def test_prefill_kernels_on_pages_of_unequal_sequences(D, block, monkeypatch):
+    """Block tables in any order, sequences of different lengths (one of them empty), norms of a wide range."""
+    n_seq, Hkv, G, q_len, longest = 4, 2, 2, 48, 300
+    per_seq = -(-longest // block)
+    g = torch.Generator(device=DEV).manual_seed(block)
+    pool = QuashKVPagedCache(n_seq * per_seq, Hkv, D, QuashKVPageConfig(key_bits=3, value_bits=3, block_size=block), device=DEV)
+    table = torch.randperm(n_seq * per_seq, generator=g, device=DEV).to(torch.int32).reshape(n_seq, per_seq)
+    k, v = _outliers(g, (n_seq, Hkv, longest, D), torch.float32), _outliers(g, (n_seq, Hkv, longest, D), torch.float32)
+    wide = 2 if D == 128 else 6                  # (the records' other kernels hold weight times norm in fp16)
+    v *= torch.logspace(-wide, wide, longest, device=DEV)[None, None, :, None]
+    pool.append_with_tables(k, v, table, torch.zeros(n_seq, dtype=torch.int32, device=DEV))
+    lens = torch.tensor([300, 0, 63, 193], dtype=torch.int32, device=DEV)
+    q = torch.randn(n_seq, Hkv * G, q_len, D, generator=g, device=DEV)
+    for causal in (False, True):
+        monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "0")
+        want = pool.attention_with_tables(q, table, lens, longest, causal=causal)
+        monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "1")
+        got = pool.attention_with_tables(q, table, lens, longest, causal=causal)
+        assert torch.equal(got[1], torch.zeros_like(got[1])) and torch.isfinite(got).all()
+        for b in (0, 2, 3):
+            assert rel_l2(got[b], want[b]) < (1e-3 if D == 128 else 5e-6), (b, causal)
