@@ -50,7 +50,6 @@ constexpr float kPiScale = 1024.f;                // entries of Pi are at most 1
 __device__ unsigned int g_prefill_timeouts = 0;
 
 template <int D, int TERMS> struct Pf {
-  static constexpr int kBlk = D / 64;                                  // 64-wide K blocks of one operand
   static constexpr int NT = (D == 128 && TERMS == 2) ? 1 : 2;          // row tiles per CTA } what 227 KB hold
   static constexpr int ST = (D == 128 && TERMS == 2) ? 1 : 2;          // token tiles in flight }
   static constexpr int kQBytes = 2 * TERMS * kRowsT * D * 2;           // [qh | wh (| ql | wl)]
@@ -116,7 +115,7 @@ __device__ __forceinline__ uint32_t half_bits2(__half a, __half b) {
 
 // ---- operand tiles ------------------------------------------------------------------------------------------------
 // Operands of the two rotations, hi and lo (B rows n, K columns k: Pi[n][k], then Pi[k][n]), and the scales of the two
-// tables.  A launch of its own: the search for the scales takes 9 us in every CTA of the kernel behind it.
+// tables.  A launch of its own: every CTA of the kernel behind it would otherwise search for the scales first.
 template <int D, int TERMS>
 __global__ void __launch_bounds__(256) prefill_setup_kernel(PrefillArgs a) {
   using P = Pf<D, TERMS>;
@@ -357,7 +356,7 @@ __device__ __forceinline__ void store_split32(uint32_t t_hi, uint32_t t_lo, cons
 template <int D, int TERMS>
 __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(PrefillArgs a) {
   using P = Pf<D, TERMS>;
-  constexpr int NT = P::NT, ST = P::ST, kBlk = P::kBlk;
+  constexpr int NT = P::NT, ST = P::ST;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* q_s = smem;                                            // [NT] query operands; first and last Pi's
   unsigned char* ring = smem + NT * P::kQBytes;
