@@ -229,7 +229,8 @@ class QuashKVPagedCache:
     # ---- data path --------------------------------------------------------------------------------
     def append(self, seq_ids: Sequence, keys: torch.Tensor, values: torch.Tensor) -> None:
         """keys, values (n_seq, num_kv_heads, new_tokens, head_size): the next ``new_tokens`` positions of
-        every listed sequence (new sequences start at position 0)."""
+        every listed sequence (new sequences start at position 0; the entries of an id that is listed more than
+        once follow one another)."""
         ops._need_cuda(keys, "QuashKVPagedCache.append")
         n, H, T, D = keys.shape
         if n != len(seq_ids) or H != self.num_kv_heads or D != self.head_size or values.shape != keys.shape:
@@ -237,12 +238,13 @@ class QuashKVPagedCache:
                              f"{self.head_size})")
         if T == 0:
             return
-        starts = np.asarray([self._lens.get(s, 0) for s in seq_ids], dtype=np.int32)
-        for s in seq_ids:
+        starts = []
+        for s in seq_ids:            # an id may be listed more than once: each entry starts where the one before it ended
+            starts.append(self._lens.get(s, 0))
             self._grow(s, T)
-            self._lens[s] = self._lens.get(s, 0) + T
+            self._lens[s] = starts[-1] + T
         table, _, _ = self.block_table(seq_ids)
-        self._store(keys, values, table, torch.from_numpy(starts).to(self.device))
+        self._store(keys, values, table, torch.tensor(starts, dtype=torch.int32, device=self.device))
 
     def append_with_tables(self, keys: torch.Tensor, values: torch.Tensor, block_table: torch.Tensor,
                            start_lens: torch.Tensor) -> None:

@@ -84,3 +84,18 @@ def test_prefill_kernels_on_pages_of_unequal_sequences(D, block, monkeypatch):
         assert torch.equal(got[1], torch.zeros_like(got[1])) and torch.isfinite(got).all()
         for b in (0, 2, 3):
             assert rel_l2(got[b], want[b]) < (1e-3 if D == 128 else 5e-6), (b, causal)
+
+
+@pytest.mark.parametrize("D,block", [(128, 16), (64, 16)])
+def test_paged_append_of_a_repeated_sequence_id(D, block):
+    """One call with an id listed twice stores what two calls with its entries one after the other store."""
+    cfg = QuashKVPageConfig(key_bits=3, value_bits=3, block_size=block)
+    k, v = (torch.randn(3, 2, 21, D, generator=torch.Generator().manual_seed(s)).to(DEV) for s in (1, 2))
+    one, two = (QuashKVPagedCache(12, 2, D, cfg, device=DEV) for _ in range(2))
+    one.append(["a", "b", "a"], k, v)
+    two.append(["a", "b"], k[:2], v[:2])
+    two.append(["a"], k[2:], v[2:])
+    for s in ("a", "b"):
+        assert one.seq_len(s) == two.seq_len(s)
+        want = two.rows_of(s)
+        assert all(torch.equal(t, want[name]) for name, t in one.rows_of(s).items())

@@ -168,6 +168,25 @@ def test_page_pool_bookkeeping_without_gpu():
         register_quashkv_backend()
 
 
+def test_paged_append_of_a_repeated_sequence_id(monkeypatch):
+    """The entries of one id go to consecutive positions of its pages, whatever stands between them in the list."""
+    from quashkv_b200.integrations.vllm_backend import QuashKVPageConfig, QuashKVPagedCache
+    monkeypatch.setattr(ops, "_need_cuda", lambda t, what: None)
+    pool = QuashKVPagedCache(8, 2, 64, QuashKVPageConfig(block_size=4), device="cpu")
+    calls = []
+    monkeypatch.setattr(pool, "_store", lambda k, v, table, starts: calls.append((table.clone(), starts.clone())))
+    ids, T = ["a", "b", "a", "a"], 3
+    x = torch.zeros(4, 2, T, 64)
+    for _ in range(2):
+        pool.append(ids, x, x)
+    assert pool.seq_len("a") == 18 and pool.seq_len("b") == 6
+    assert calls[0][1].tolist() == [0, 0, 3, 6] and calls[1][1].tolist() == [9, 3, 12, 15]
+    for table, starts in calls:
+        assert starts.dtype == torch.int32 and table.dtype == torch.int32
+        slots = [(int(table[i, p // 4]), p % 4) for i in range(4) for p in range(int(starts[i]), int(starts[i]) + T)]
+        assert len(set(slots)) == len(slots)              # no position is written twice
+
+
 def test_index_file_checks_without_gpu(tmp_path):
     """An empty index round-trips on CPU; foreign or inconsistent files are refused."""
     qk.QuashIndex(64, 4, seed=7).save(tmp_path / "empty.pt")
