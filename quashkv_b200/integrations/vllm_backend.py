@@ -236,7 +236,7 @@ class QuashKVPagedCache:
         if n != len(seq_ids) or H != self.num_kv_heads or D != self.head_size or values.shape != keys.shape:
             raise ValueError(f"Expected keys and values of shape ({len(seq_ids)}, {self.num_kv_heads}, T, "
                              f"{self.head_size})")
-        if T == 0:
+        if n == 0 or T == 0:
             return
         starts = []
         for s in seq_ids:            # an id may be listed more than once: each entry starts where the one before it ended

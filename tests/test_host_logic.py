@@ -185,6 +185,8 @@ def test_paged_append_of_a_repeated_sequence_id(monkeypatch):
         assert starts.dtype == torch.int32 and table.dtype == torch.int32
         slots = [(int(table[i, p // 4]), p % 4) for i in range(4) for p in range(int(starts[i]), int(starts[i]) + T)]
         assert len(set(slots)) == len(slots)              # no position is written twice
+    pool.append([], torch.zeros(0, 2, T, 64), torch.zeros(0, 2, T, 64))        # a step without sequences stores nothing
+    assert len(calls) == 2
 
 
 def test_index_file_checks_without_gpu(tmp_path):
