@@ -24,7 +24,8 @@
 // of 128 at 3/3 bits, 3016 -> 991 us; error against 64 bits with TERMS = 2 0.70 to 0.97 of the fp32 kernel's over ten
 // shapes.  Bound by the softmax warps' chain (tensor memory reads, 1.8 instructions a cycle); the tensor pipe is 20 % busy.
 //
-// Every wait is bounded; one that runs out ends the use of the tensor core in its CTA and is counted.
+// Every wait is bounded; one that runs out is counted and ends the use of the tensor core in its CTA, whose rows are then
+// attended in fp32 on the CUDA cores (attend_rows_fp32).
 #include <math.h>
 #include <stdlib.h>
 
@@ -86,6 +87,8 @@ struct PrefillArgs {
   float* norms;
   float* tab;                // [0] key table scale, [1] value table scale, [2] 0, or NaN for a table that the records do not cover
   int tiles;                 // token tiles per (batch, kv head)
+  int test_drop_mma;         // test hook: the first CTA issues nothing for its second token tile, so that the waits on it
+                             // run out and its rows come from the fp32 way out
 };
 
 // 2^(K - e) for a magnitude 2^e <= x < 2^(e+1): x times it lies in [2^K, 2^(K+1)).  Always a normal number, and so is
@@ -157,6 +160,44 @@ __global__ void __launch_bounds__(256) prefill_setup_kernel(PrefillArgs a) {
   }
 }
 
+// Coordinates 16 g .. of token `tok` as the cache holds them: key codes (a.wk bits each), sign bits, value codes (a.wv
+// bits each) and the token's norms.
+template <int D>
+__device__ __forceinline__ void load_group16(const PrefillArgs& a, int seg, int b, int hkv, int64_t tok, int g,
+                                             uint64_t& kbits, uint64_t& vbits, uint32_t& sbits, float& kn, float& vn) {
+  int64_t unit = 0;                            // pages: the block, and the token inside it
+  int off = 0;
+  if (a.block_table) {
+    const unsigned u = static_cast<unsigned>(tok), bs = static_cast<unsigned>(a.block_size);
+    unit = static_cast<int64_t>(a.block_table[static_cast<int64_t>(b) * a.max_blocks + u / bs]) * a.Hkv + hkv;
+    off = static_cast<int>(u % bs);
+  }
+  if (a.records) {
+    const int64_t r = a.block_table ? unit * (a.block_size >> 4) + (off >> 4)
+                                    : static_cast<int64_t>(seg) * (a.cache.capacity >> 4) + (tok >> 4);
+    const uint8_t* rec = a.records + r * tile::kBytes;
+    const int k = static_cast<int>(tok & 15);
+    kbits = *reinterpret_cast<const uint32_t*>(rec + tile::key_code_offset(k, g));
+    sbits = *reinterpret_cast<const uint32_t*>(rec + tile::key_sign_offset(k, g >> 1)) >> (16 * (g & 1));
+    uint32_t w[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      w[i] = *reinterpret_cast<const uint32_t*>(rec + tile::val_word_offset(tile::val_lane(k, g), 3 * tile::val_group(k) + i));
+    vbits = tile::gather_codes16(w, tile::val_half_shift(k));
+    kn = *reinterpret_cast<const float*>(rec + tile::key_norm_offset(k));
+    vn = *reinterpret_cast<const float*>(rec + tile::val_norm_offset(k));
+  } else {
+    const int64_t row = a.block_table ? unit * a.block_size + off : static_cast<int64_t>(seg) * a.cache.capacity + tok;
+    const uint16_t* kp = reinterpret_cast<const uint16_t*>(a.cache.k_codes + row * (D / 8 * a.wk)) + g * a.wk;
+    const uint16_t* vp = reinterpret_cast<const uint16_t*>(a.cache.v_codes + row * (D / 8 * a.wv)) + g * a.wv;
+    for (int i = 0; i < a.wk; ++i) kbits |= static_cast<uint64_t>(kp[i]) << (16 * i);
+    for (int i = 0; i < a.wv; ++i) vbits |= static_cast<uint64_t>(vp[i]) << (16 * i);
+    sbits = reinterpret_cast<const uint16_t*>(a.cache.k_signs + row * (D / 8))[g];
+    kn = a.cache.k_norms[row];
+    vn = a.cache.v_norms[row];
+  }
+}
+
 // Tile, segment per CTA: 64 tokens, four threads each.  Codes go through shared memory as bytes, and leave as 16-byte
 // chunks of eight fp16 in the swizzled operand order.  Bound by the writes (768 to 1280 bytes a token at d = 128), which stay in L2 for the kernel behind it.
 template <int D, int TERMS>
@@ -190,39 +231,7 @@ __global__ void __launch_bounds__(256) prefill_operands_kernel(PrefillArgs a) {
     uint32_t sbits = 0;
     float kn = 0.f, vn = 0.f;
     const bool live = tok < kv_len;
-    if (live) {
-      int64_t unit = 0;                            // pages: the block, and the token inside it
-      int off = 0;
-      if (a.block_table) {
-        const unsigned u = static_cast<unsigned>(tok), bs = static_cast<unsigned>(a.block_size);
-        unit = static_cast<int64_t>(a.block_table[static_cast<int64_t>(b) * a.max_blocks + u / bs]) * a.Hkv + hkv;
-        off = static_cast<int>(u % bs);
-      }
-      if (a.records) {
-        const int64_t r = a.block_table ? unit * (a.block_size >> 4) + (off >> 4)
-                                        : static_cast<int64_t>(seg) * (a.cache.capacity >> 4) + (tok >> 4);
-        const uint8_t* rec = a.records + r * tile::kBytes;
-        const int k = static_cast<int>(tok & 15);
-        kbits = *reinterpret_cast<const uint32_t*>(rec + tile::key_code_offset(k, g));
-        sbits = *reinterpret_cast<const uint32_t*>(rec + tile::key_sign_offset(k, g >> 1)) >> (16 * (g & 1));
-        uint32_t w[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-          w[i] = *reinterpret_cast<const uint32_t*>(rec + tile::val_word_offset(tile::val_lane(k, g), 3 * tile::val_group(k) + i));
-        vbits = tile::gather_codes16(w, tile::val_half_shift(k));
-        kn = *reinterpret_cast<const float*>(rec + tile::key_norm_offset(k));
-        vn = *reinterpret_cast<const float*>(rec + tile::val_norm_offset(k));
-      } else {
-        const int64_t row = a.block_table ? unit * a.block_size + off : static_cast<int64_t>(seg) * a.cache.capacity + tok;
-        const uint16_t* kp = reinterpret_cast<const uint16_t*>(a.cache.k_codes + row * (D / 8 * a.wk)) + g * a.wk;
-        const uint16_t* vp = reinterpret_cast<const uint16_t*>(a.cache.v_codes + row * (D / 8 * a.wv)) + g * a.wv;
-        for (int i = 0; i < a.wk; ++i) kbits |= static_cast<uint64_t>(kp[i]) << (16 * i);
-        for (int i = 0; i < a.wv; ++i) vbits |= static_cast<uint64_t>(vp[i]) << (16 * i);
-        sbits = reinterpret_cast<const uint16_t*>(a.cache.k_signs + row * (D / 8))[g];
-        kn = a.cache.k_norms[row];
-        vn = a.cache.v_norms[row];
-      }
-    }
+    if (live) load_group16<D>(a, seg, b, hkv, tok, g, kbits, vbits, sbits, kn, vn);
     const uint32_t km = (1u << a.wk) - 1u, vm = (1u << a.wv) - 1u;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -349,6 +358,81 @@ __device__ __forceinline__ void store_split32(uint32_t t_hi, uint32_t t_lo, cons
   }
   umma::tmem_st16(t_hi, hi);
   if (with_lo) umma::tmem_st16(t_lo, lo);
+}
+
+// Query rows first .. first + 31 of a segment, one after another, in fp32 on the CUDA cores straight from the cache: the
+// way out of a CTA in which a wait ran out.  A warp per row, a lane its coordinates lane, lane + 32, ...; far slower than
+// the tensor core, and written only to be right.
+template <int D>
+__device__ __forceinline__ void attend_rows_fp32(const PrefillArgs& a, int seg, int b, int hkv, int64_t kv_len, int first,
+                                                 int nq, int lane) {
+  constexpr int PL = D / 32;
+  const uint32_t km = (1u << a.wk) - 1u, vm = (1u << a.wv) - 1u;
+  auto times = [&](const float (&x)[PL], bool transposed, float (&y)[PL]) {      // y = Pi x, or its transpose
+#pragma unroll
+    for (int t = 0; t < PL; ++t) y[t] = 0.f;
+#pragma unroll
+    for (int u = 0; u < PL; ++u) {
+#pragma unroll 1
+      for (int j = 0; j < 32; ++j) {
+        const float xj = __shfl_sync(QKV_FULL_MASK, x[u], j);
+        const int from = 32 * u + j;
+#pragma unroll
+        for (int t = 0; t < PL; ++t) {
+          const int to = lane + 32 * t;
+          y[t] = fmaf(xj, __ldg(a.Pi + (transposed ? from * D + to : to * D + from)), y[t]);
+        }
+      }
+    }
+  };
+#pragma unroll 1
+  for (int r = first; r < first + 32 && r < nq; ++r) {
+    const int64_t qrow = (static_cast<int64_t>(b) * a.Hq + hkv * a.G) * a.q_len + r;
+    const int64_t lim = a.causal ? kv_len - a.q_len + r % a.q_len : kv_len - 1;
+    float x[PL], y[PL], w[PL], o[PL], m = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int t = 0; t < PL; ++t) x[t] = load_float(a.q, a.q_dtype, qrow * D + lane + 32 * t);
+    times(x, false, y);
+#pragma unroll
+    for (int t = 0; t < PL; ++t) {
+      w[t] = (a.qjl_scale * a.scale) * (fabsf(y[t]) * __ldg(a.S + lane + 32 * t));
+      y[t] *= a.scale;
+      o[t] = 0.f;
+    }
+#pragma unroll 1
+    for (int64_t tok = 0; tok <= lim; ++tok) {
+      float s = 0.f, vc[PL], kn = 0.f, vn = 0.f;
+#pragma unroll
+      for (int t = 0; t < PL; ++t) {
+        uint64_t kbits = 0, vbits = 0;
+        uint32_t sbits = 0;
+        const int j = lane + 32 * t, c = j & 15;
+        load_group16<D>(a, seg, b, hkv, tok, j >> 4, kbits, vbits, sbits, kn, vn);
+        s = fmaf(y[t], __ldg(a.kcent + (static_cast<uint32_t>(kbits >> (c * a.wk)) & km)), s) + ((sbits >> c) & 1u ? w[t] : -w[t]);
+        vc[t] = __ldg(a.vcent + (static_cast<uint32_t>(vbits >> (c * a.wv)) & vm));
+      }
+#pragma unroll
+      for (int e = 16; e > 0; e >>= 1) s += __shfl_xor_sync(QKV_FULL_MASK, s, e);
+      s *= kn;
+      if (s > m) {
+        const float alpha = m == -INFINITY ? 0.f : expf(m - s);
+        m = s;
+        l *= alpha;
+#pragma unroll
+        for (int t = 0; t < PL; ++t) o[t] *= alpha;
+      }
+      const float p = s == -INFINITY ? 0.f : expf(s - m), pv = p * vn;
+      l += p;
+#pragma unroll
+      for (int t = 0; t < PL; ++t) o[t] = fmaf(pv, vc[t], o[t]);
+    }
+    const float inv = 1.f / fmaxf(l, 1e-30f);
+#pragma unroll
+    for (int t = 0; t < PL; ++t) o[t] *= inv;
+    times(o, true, y);
+#pragma unroll
+    for (int t = 0; t < PL; ++t) a.out[qrow * D + lane + 32 * t] = y[t] + a.tab[2];
+  }
 }
 
 // Warps 0..3 own row tile 0, warps 4..7 row tile 1 (NT = 2): a thread per query row.  Of the four warps behind them one
@@ -548,6 +632,7 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
         for (int t = 0; t < NT && ok; ++t) {
           if (!(ok = wait(p_ready + t, j & 1))) break;
           if (t == 0 && !(ok = wait(v_full + j % ST, (j / ST) & 1))) break;
+          if (a.test_drop_mma && (blockIdx.x | blockIdx.y) == 0 && t == 0 && j == 1) continue;   // test hook
           umma::fence_after_sync();
           values(t, j);
           if (t == NT - 1) umma::commit(v_free + j % ST);
@@ -827,6 +912,7 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
         }
       }
     }
+    if (!ok) attend_rows_fp32<D>(a, seg, b, hkv, kv_len, r0 + 32 * warp, nq, lane);       // warp-uniform
   }
   umma::fence_before_sync();
   __syncthreads();
@@ -909,6 +995,8 @@ int launch_prefill(const AttnArgs& s, const void* q, int q_dtype, int key_bits, 
   a.wk = key_bits - 1; a.wv = val_bits; a.kv_len = s.kv_len;
   a.Pi = s.Pi; a.S = S; a.kcent = s.kcent; a.vcent = s.vcent; a.qjl_scale = qjl_scale; a.scale = scale;
   a.out = s.out;
+  const char* hook = getenv("QUASHKV_B200_TEST_DROP_MMA");      // 1: tests only
+  a.test_drop_mma = hook && hook[0] == '1';
   a.img = static_cast<unsigned char*>(workspace);
   if (s.d == 64) return launch_t<64, 2>(a, st);
   return s.records ? launch_t<128, 1>(a, st) : launch_t<128, 2>(a, st);
