@@ -10,8 +10,9 @@
 //   scores     [q | w] x [centroid | +-1], K = 2 D, accumulated in tensor memory
 //   softmax    a thread per query row, log2 domain, reference exponent rounded up to a whole number, so that every
 //              rescaling is by a power of two and exact
-//   values     weights times value norm as the A operand in tensor memory, centroids transposed as B; the sum of a tile
-//              is added to fp32 registers, so no accumulator is rescaled and none truncates over a long sequence
+//   values     weights times value norm, scaled by a power of two, as the A operand in tensor memory, centroids transposed
+//              as B; the sum of a tile is added to fp32 registers, so no accumulator is rescaled and none truncates over a
+//              long sequence
 //   un-rotation  (sum / l) @ Pi, as MMAs, straight to the output rows
 // Two row tiles share each token tile: the tensor core works on one while the other's softmax runs.
 //
@@ -40,7 +41,8 @@ namespace {
 
 constexpr int kTok = 64;                          // tokens per tile
 constexpr int kRowsT = 128;                       // query rows per row tile = MMA M
-constexpr int kNormBytes = (2 * kTok + 4) * 4;    // key norms, value norms x 2^s, 2^-s, padding
+// Norms of a tile: of keys, of values (TERMS = 1: x 2^s, then 2^-s, padding, and a byte of further scale per token).
+constexpr int kNormBytes = (2 * kTok + 4) * 4 + kTok;
 constexpr int kNormSlots = 4;
 // The tensor core truncates its fp32 sums, so that results come out small by 2e-7 to 5e-7 (slope against 64-bit results
 // over 16 shapes, mean 3.2e-7; the fp32 kernel's is below 3e-8).  3 * 2^-23 takes the mean back with TERMS = 2: the error
@@ -282,14 +284,25 @@ __global__ void __launch_bounds__(256) prefill_operands_kernel(PrefillArgs a) {
     if (TERMS == 2) *reinterpret_cast<uint4*>(dst + kOp) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
   if (tid < 32) {
-    // value norms leave scaled by a power of two that brings the tile's largest to [2^13, 2^14): whatever their range,
-    // weight times norm stays inside fp16, and a weight of 2^-28 still is a normal number there
     const float v0 = nrm_s[1][tid], v1 = nrm_s[1][tid + 32];
-    float mx = fmaxf(fabsf(v0), fabsf(v1));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(QKV_FULL_MASK, mx, o));
-    const float down = scale_to<13>(mx);
     float* nb = a.norms + tile_idx * (kNormBytes / 4);
+    float down = 1.f;
+    if (TERMS == 1) {
+      // weights times norms become single fp16 numbers: the norms leave scaled by a power of two that brings the tile's
+      // largest to [2^14, 2^15), so that the product stays inside fp16 and is a normal number down to 2^-28 of it.  A row
+      // that sees only tokens 0 .. e of the tile scales up further, by 2^(byte e).  (TERMS = 2: every row for itself.)
+      float p0 = fabsf(v0), p1 = fabsf(v1);                             // largest norm of tokens 0 .. tid, 32 .. tid + 32
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float q0 = __shfl_up_sync(QKV_FULL_MASK, p0, o), q1 = __shfl_up_sync(QKV_FULL_MASK, p1, o);
+        if (tid >= o) { p0 = fmaxf(p0, q0); p1 = fmaxf(p1, q1); }
+      }
+      p1 = fmaxf(p1, __shfl_sync(QKV_FULL_MASK, p0, 31));
+      down = scale_to<14>(__shfl_sync(QKV_FULL_MASK, p1, 31));
+      uint8_t* up = reinterpret_cast<uint8_t*>(nb + 2 * kTok + 4);
+      up[tid] = static_cast<uint8_t>((__float_as_uint(scale_to<14>(p0 * down)) >> 23) - 127u);
+      up[tid + 32] = static_cast<uint8_t>((__float_as_uint(scale_to<14>(p1 * down)) >> 23) - 127u);
+    }
     nb[tid] = nrm_s[0][tid];
     nb[tid + 32] = nrm_s[0][tid + 32];
     nb[kTok + tid] = v0 * down;
@@ -345,7 +358,16 @@ __device__ __forceinline__ void load32(const void* q, int dtype, int64_t idx, bo
   }
 }
 
-// Sixteen tensor-memory columns of hi and of lo from 32 values v * s.
+// v *= s, two at a time.
+__device__ __forceinline__ void scale32(float (&v)[32], float s) {
+#pragma unroll
+  for (int e = 0; e < 32; e += 2)
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\t"
+        "mul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}\n"
+        : "+f"(v[e]), "+f"(v[e + 1]) : "f"(s));
+}
+
+// Sixteen tensor-memory columns of hi and of lo from 32 values.
 __device__ __forceinline__ void store_split32(uint32_t t_hi, uint32_t t_lo, const float (&v)[32], bool with_lo) {
   uint32_t hi[16], lo[16];
 #pragma unroll
@@ -435,6 +457,26 @@ __device__ __forceinline__ void attend_rows_fp32(const PrefillArgs& a, int seg, 
   }
 }
 
+// Query rows of a CTA: rows first .. of a segment (batch entry b, KV head hkv), late positions (more tokens) first.
+struct CtaRows { int seg, b, hkv, first; int64_t kv_len; };
+template <int D, int TERMS>
+__device__ __forceinline__ CtaRows cta_rows(const PrefillArgs& a, uint32_t bx, uint32_t by) {
+  constexpr int kRows = Pf<D, TERMS>::NT * kRowsT;
+  CtaRows r;
+  r.seg = static_cast<int>(bx);
+  r.b = r.seg / a.Hkv;
+  r.hkv = r.seg % a.Hkv;
+  int rt = static_cast<int>(gridDim.y - 1 - by);
+  if (a.causal && a.q_len % kRows == 0) {                               // ... over all heads of the segment
+    const int per_head = a.q_len / kRows;
+    rt = (static_cast<int>(by) % a.G) * per_head + per_head - 1 - static_cast<int>(by) / a.G;
+  }
+  r.first = rt * kRows;
+  r.kv_len = a.kv_len;
+  if (a.block_table) r.kv_len = min(static_cast<int64_t>(max(a.seq_lens[r.b], 0)), a.kv_len);
+  return r;
+}
+
 // Warps 0..3 own row tile 0, warps 4..7 row tile 1 (NT = 2): a thread per query row.  Of the four warps behind them one
 // thread issues every MMA and one every copy.  
 template <int D, int TERMS>
@@ -462,16 +504,9 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-  // ---- which rows ----
-  const int nq = a.G * a.q_len, seg = blockIdx.x, b = seg / a.Hkv, hkv = seg % a.Hkv;
-  int rt = static_cast<int>(gridDim.y - 1 - blockIdx.y);                // late positions (more tokens) first
-  if (a.causal && a.q_len % (NT * kRowsT) == 0) {                       // ... over all heads of the segment
-    const int per_head = a.q_len / (NT * kRowsT);
-    rt = (static_cast<int>(blockIdx.y) % a.G) * per_head + per_head - 1 - static_cast<int>(blockIdx.y) / a.G;
-  }
-  const int r0 = rt * NT * kRowsT;
-  int64_t kv_len = a.kv_len;
-  if (a.block_table) kv_len = min(static_cast<int64_t>(max(a.seq_lens[b], 0)), a.kv_len);
+  const CtaRows rows = cta_rows<D, TERMS>(a, blockIdx.x, blockIdx.y);
+  const int nq = a.G * a.q_len, seg = rows.seg, b = rows.b, hkv = rows.hkv, r0 = rows.first;
+  const int64_t kv_len = rows.kv_len;
   int64_t seen = kv_len;
   if (a.causal) {
     const int n_rows = nq - r0 < NT * kRowsT ? nq - r0 : NT * kRowsT, p_first = r0 % a.q_len;
@@ -846,29 +881,51 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
         }
       };
       const uint32_t pt = my + 64 * (j % P::SB);
+      float up;
       if (P::kSplit) {                    // hi to columns 0 .. 31 of the scores' place, lo to 32 .. 63: read all of it first
+        // the row's products are scaled by a power of two that brings their largest to [2^14, 2^15): what another token
+        // weighs, or a token that this row cannot see, takes no bits from them
         uint32_t v[2][32];
+        float pv[2][32], mp[2] = {0.f, 0.f};
         scores32(j, 0, v[0]);
         scores32(j, 32, v[1]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          float pv[32];
-          weigh(32 * h, v[h], pv);
-          store_split32(pt + 16 * h, pt + 32 + 16 * h, pv, true);
+          weigh(32 * h, v[h], pv[h]);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) mp[e & 1] = fmaxf(mp[e & 1], fabsf(pv[h][e]));
+        }
+        const float down = scale_to<14>(fmaxf(mp[0], mp[1]));
+        up = inverse_pow2(down);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          scale32(pv[h], down);
+          store_split32(pt + 16 * h, pt + 32 + 16 * h, pv[h], true);
         }
       } else {                            // hi alone stays inside the half that has been read
+        // the tile's scale is that of its largest norm; a row that sees only a part of the tile takes the part's
+        float more = 1.f;
+        if (masked && left >= 0) {
+          const uint32_t k = reinterpret_cast<const uint8_t*>(nb + 2 * kTok + 4)[left < kTok ? left : kTok - 1];
+          more = __uint_as_float((127u + k) << 23);
+        }
+        up = nb[2 * kTok] * inverse_pow2(more);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t v[32];
           float pv[32];
           scores32(j, 32 * h, v);
           weigh(32 * h, v, pv);
+          if (masked) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) pv[e] *= more;
+          }
           store_split32(pt + 16 * h, pt, pv, false);
         }
       }
       l = l * alpha + ((ls[0] + ls[1]) + (ls[2] + ls[3]));
       alpha_prev = alpha;
-      up_prev = nb[2 * kTok];
+      up_prev = up;
       umma::tmem_st_wait();
       umma::fence_before_sync();
       arrive(p_ready + t);
@@ -912,7 +969,13 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
         }
       }
     }
-    if (!ok) attend_rows_fp32<D>(a, seg, b, hkv, kv_len, r0 + 32 * warp, nq, lane);       // warp-uniform
+    if (!ok) {                              // warp-uniform
+      uint32_t bx, by, th;                  // (read again: nothing of this is held in registers through the loop)
+      asm volatile("mov.u32 %0, %%ctaid.x;\n\tmov.u32 %1, %%ctaid.y;\n\tmov.u32 %2, %%tid.x;\n" : "=r"(bx), "=r"(by), "=r"(th));
+      const CtaRows c = cta_rows<D, TERMS>(a, bx, by);
+      attend_rows_fp32<D>(a, c.seg, c.b, c.hkv, c.kv_len, c.first + static_cast<int>(th & ~31u), a.G * a.q_len,
+                          static_cast<int>(th & 31u));
+    }
   }
   umma::fence_before_sync();
   __syncthreads();

@@ -20,6 +20,38 @@ def ulp_diff(a: torch.Tensor, b: torch.Tensor) -> int:
     return int((ia - ib).abs().max()) if ia.numel() else 0
 
 
+def attention_64(engine, queries, causal: bool) -> torch.Tensor:
+    """What ``engine.attention`` stands for (reference engine.py:204-299), in 64 bits from its stored codes: scores
+    k_norm (q_rot . c_K + qjl_scale |q_rot| . S sign), softmax, values v_norm c_V un-rotated."""
+    import quashkv_b200 as qk
+    p, n = engine.row_planes(), engine.total_tokens
+    B, Hq, Q, D = queries.shape
+    dev, kq, vq = queries.device, engine.key_quantizer, engine.value_quantizer
+    f64 = lambda t: t.to(dev).double()      # noqa: E731
+    unpack = lambda name, bits: qk.unpack_bits(p[name].contiguous(), bits, D).reshape(B, -1, n, D)      # noqa: E731
+    Pi, S = f64(kq.mse_quantizer.Pi), f64(kq.S).reshape(-1)
+    keys = f64(kq.mse_quantizer.codebook.centroids)[unpack("k_codes", engine.key_bits - 1).long()]
+    signs = (2.0 * unpack("k_signs", 1).double() - 1.0) * S
+    vals = f64(vq.codebook.centroids)[unpack("v_codes", engine.value_bits).long()] @ f64(vq.Pi)
+    kn, vn = (f64(p[name].contiguous()).reshape(B, -1, n) for name in ("k_norms", "v_norms"))
+    G = Hq // keys.shape[1]
+    hidden = torch.arange(n, device=dev)[None] > n - Q + torch.arange(Q, device=dev)[:, None]
+    out = torch.empty(B, Hq, Q, D, dtype=torch.float64, device=dev)
+    for b in range(B):
+        for h in range(Hq):
+            x, s = f64(queries[b, h]) @ Pi.T, h // G
+            score = (x @ keys[b, s].T + kq.qjl_scale * (x.abs() @ signs[b, s].T)) * kn[b, s] / D ** 0.5
+            if causal:
+                score = score.masked_fill(hidden, float("-inf"))
+            out[b, h] = torch.softmax(score, -1) @ (vals[b, s] * vn[b, s][:, None])
+    return out
+
+
+def row_errors(got: torch.Tensor, want: torch.Tensor) -> torch.Tensor:
+    """Relative error of every row (last dimension), flat."""
+    return ((got.double() - want).norm(dim=-1) / want.norm(dim=-1).clamp(min=1e-300)).flatten()
+
+
 def code_ties(x, Pi, tables, got, want, kind="code", centroids=None, S=None, codes_for_resid=None):
     """Explain every mismatch between two code tensors as a tie.
 

@@ -6,7 +6,7 @@ import torch
 import quashkv_b200 as qk
 from quashkv_b200 import _lib
 from quashkv_b200.integrations.vllm_backend import QuashKVPageConfig, QuashKVPagedCache
-from helpers import rel_l2
+from helpers import attention_64, rel_l2, row_errors
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -134,3 +134,27 @@ def test_prefill_rows_are_right_after_a_wait_that_ran_out(D, bits, paged, monkey
         assert rel_l2(got, want) < bound and rel_l2(got[0], want[0]) < bound
         assert torch.equal(got[1], plain[1]) and not torch.equal(got[0], plain[0])
         assert torch.equal(attend(causal), plain)
+
+
+@pytest.mark.parametrize("log2_step", [10, 20, 34, 60])
+@pytest.mark.parametrize("D,bits", [(64, 3), (64, 4), (128, 4), (128, 3)])
+def test_prefill_keeps_rows_beside_a_much_larger_value_norm(D, bits, log2_step, monkeypatch):
+    """The last token of every 64 has value norms 2^step times the others': each row for itself, before and after it
+    sees one.  fp32 arithmetic keeps a row to about 3e-6 whatever the norms, and so do hi + lo operands scaled per row.
+    At d = 128, 3/3 bits a weight times a norm is one fp16 number, normal down to 2^-28 of the tile's largest norm that
+    the row sees (roundings of 2^-12 to queries, tables and products: below 3e-3 a row); a neighbour that is in sight,
+    2^34 larger and weighs nothing is beyond that, so those steps are checked on the rows of the first tile, which see
+    none."""
+    n = 130
+    g = torch.Generator(device=DEV).manual_seed(D + log2_step)
+    k, v = (_outliers(g, (1, 2, n, D), torch.float32) for _ in range(2))
+    v[:, :, 63::64] *= 2.0 ** log2_step
+    q = torch.randn(1, 4, n, D, generator=g, device=DEV)
+    eng = qk.QuashKVEngine(D, bits, bits, seed=42, device=DEV, pack_storage=True)
+    eng.append(k, v)
+    monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "1")
+    err = row_errors(eng.attention(q, causal=True), attention_64(eng, q, True)).reshape(4, n)
+    if (D, bits) != (128, 3):
+        assert float(err.max()) < 1e-5
+    else:
+        assert float(err[:, :63].max()) < 3e-3 and (log2_step > 24 or float(err.max()) < 3e-3)
