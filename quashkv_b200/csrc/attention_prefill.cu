@@ -19,11 +19,12 @@
 // Precision.  Every operand that does not fit fp16 goes in as hi + lo (22 bits, scaled per row or per table by powers of
 // two), with the products lo x hi, hi x lo, hi x hi, smallest first.  That holds for both rotations always, and for all
 // of scores and values with TERMS = 2 (every width but the 3/3-bit records of d = 128, whose other kernels round
-// queries, tables and weights to fp16 once as well: TERMS = 1).
+// queries, tables and weights to fp16 once as well: TERMS = 1).  Error against 64-bit results: with TERMS = 2 0.71 of the
+// fp32 kernel's on average over 34 shapes, 0.93 at the worst of them; with TERMS = 1 that of the kernels it stands beside.
 //
-// Measured (before: the decode kernels): 8 x 1024 causal tokens, 32 / 4 heads of 64, 8609 -> 491 us; 2 x 4096, 32 / 8 heads
-// of 128 at 3/3 bits, 3016 -> 991 us; error against 64 bits with TERMS = 2 0.70 to 0.97 of the fp32 kernel's over ten
-// shapes.  Bound by the softmax warps' chain (tensor memory reads, 1.8 instructions a cycle); the tensor pipe is 20 % busy.
+// Measured (before: the decode kernels): 8 x 1024 causal tokens, 32 / 4 heads of 64, 8609 -> 500 us; 2 x 4096, 32 / 8 heads
+// of 128 at 3/3 bits, 3016 -> 1000 us.  Bound by the softmax warps' chain (tensor memory reads, 1.8 instructions a cycle);
+// the tensor pipe is 20 % busy.
 //
 // Every wait is bounded; one that runs out is counted and ends the use of the tensor core in its CTA, whose rows are then
 // attended in fp32 on the CUDA cores (attend_rows_fp32).
@@ -44,10 +45,13 @@ constexpr int kRowsT = 128;                       // query rows per row tile = M
 // Norms of a tile: of keys, of values (TERMS = 1: x 2^s, then 2^-s, padding, and a byte of further scale per token).
 constexpr int kNormBytes = (2 * kTok + 4) * 4 + kTok;
 constexpr int kNormSlots = 4;
-// The tensor core truncates its fp32 sums, so that results come out small by 2e-7 to 5e-7 (slope against 64-bit results
-// over 16 shapes, mean 3.2e-7; the fp32 kernel's is below 3e-8).  3 * 2^-23 takes the mean back with TERMS = 2: the error
-// against 64 bits is then below the fp32 kernel's at each of those shapes, without it up to a fifth above.
-constexpr float kUntruncate = 1.f + 3.f / 8388608.f;
+// The tensor core truncates: an MMA that adds to an accumulator drops what lies below its last bit, on average half a
+// unit towards zero, which is 2^-24 E[1 / m] = 2^-24 / (2 ln 2) of a value with mantissa m.  A sum of s like steps is
+// truncated at 1/s, 2/s, ... of itself, so it comes out small by (s + 1) / 2 of that.  With TERMS = 2 the factors that
+// follow a sum anyway (score units, inverse scales) carry the expected loss of the steps in front of them; it follows from
+// the number of steps alone.  Mean slope against 64-bit results over 34 shapes: -2.5e-7 without it, 1e-8 with it.
+constexpr double kDrop = 0.72134752 / 16777216.0;
+constexpr double steps_lost(int s) { return 0.5 * (s + 1); }
 constexpr float kPiScale = 1024.f;                // entries of Pi are at most 1: hi and lo both far from subnormals
 
 __device__ unsigned int g_prefill_timeouts = 0;
@@ -70,6 +74,14 @@ template <int D, int TERMS> struct Pf {
   static constexpr int SB = kSplit ? 1 : 2;                            // score tiles in flight
   static constexpr int kO2 = D == 64 ? 192 : 384;
   static constexpr int kR1 = D == 64 ? 64 : 256, kR2 = D == 64 ? 192 : 384;
+  // Steps of 16 of the parts of a sum, and what truncation takes of it, in kDrop.
+  static constexpr int kS = D / 16, kA = kSplit ? kS / 4 : kS, kB = kSplit ? kS / 2 + kS / 8 : kS;      // rotations: 0, kA, kB, kS
+  static constexpr int kScorePart = D == 64 ? D / 16 : D / 32;
+  static constexpr int kValuePart = kTok / 32;
+  static constexpr double kRotLost =
+      (kA * steps_lost(kA) + (kB - kA) * steps_lost(kB - kA) + (kS - kB) * steps_lost(kS - kB)) / kS;
+  static constexpr double kScoresUp = kSplit ? 1.0 + kDrop * (kRotLost + steps_lost(kScorePart)) : 1.0;
+  static constexpr double kOutputUp = kSplit ? 1.0 + kDrop * (kRotLost + steps_lost(kValuePart)) : 1.0;
   static constexpr int kThreads = NT * kRowsT + 128;
   static constexpr size_t kSmem = static_cast<size_t>(NT) * kQBytes + ST * kTileBytes + kNormSlots * kNormBytes + 256;
   static_assert(kPiBytes <= NT * kQBytes, "the rotation's operand uses the queries' place");
@@ -587,7 +599,7 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
         auto step = [&](uint32_t dst, uint32_t av, uint32_t bv, int ks, bool acc) {
           umma::mma_f16_ts(dst, av + 8 * ks, umma::smem_desc_sw128(bv + (ks >> 2) * (D * 128) + (ks & 3) * 32), id_d, acc);
         };
-        constexpr int kS = D / 16, kA = P::kSplit ? kS / 4 : kS, kB = P::kSplit ? kS / 2 + kS / 8 : kS;
+        constexpr int kS = P::kS, kA = P::kA, kB = P::kB;
 #pragma unroll
         for (int ks = 0; ks < kS; ++ks) step(d, al, pi_addr, ks, ks != 0);
 #pragma unroll
@@ -609,7 +621,7 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
           }
         };
         if (P::kSplit) {
-          constexpr int kH = D == 64 ? D / 16 : D / 32;                        // k-steps of a part
+          constexpr int kH = P::kScorePart;
           const uint32_t sign = D == 64 ? d + 64 : d + 256;
           product(d, 2, 0, 0, D / 16, false);                                  // ql ch
           product(d, 0, 2, 0, D / 16, true);                                   // qh cl
@@ -635,9 +647,9 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
           const uint32_t av = pr == 0 ? pl : ph, bv = va + (pr == 1 ? kTok * D * 2 : 0);
 #pragma unroll
           for (int ks = 0; ks < kTok / 16; ++ks) {
-            const bool second = P::kSplit && pr == 2 && ks >= 2;
+            const bool second = P::kSplit && pr == 2 && ks >= P::kValuePart;
             umma::mma_f16_ts(second ? base + P::kO2 : d, av + 8 * ks, umma::smem_desc_sw128(bv + ks * 32), id_d,
-                             second ? ks != 2 : acc);
+                             second ? ks != P::kValuePart : acc);
             acc = true;
           }
         }
@@ -701,7 +713,7 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
     int64_t lim64 = -1;                     // last token this row sees
     if (live) lim64 = a.causal ? kv_len - a.q_len + r % a.q_len : kv_len - 1;
     const int lim = lim64 < -1 ? -1 : static_cast<int>(lim64);
-    constexpr float kLog2e = 1.4426950408889634f;
+    constexpr float kLog2e = static_cast<float>(1.4426950408889634 * P::kScoresUp);
 
     auto rotated32 = [&](int c, uint32_t (&v)[32]) {        // 32 columns of a rotation's result
       umma::tmem_ld32(my + c, v);
@@ -954,7 +966,7 @@ __global__ void __launch_bounds__(Pf<D, TERMS>::kThreads, 1) prefill_kernel(Pref
       ok = wait_all(out_full + t, 0);
       umma::fence_after_sync();
       if (ok) {
-        const float un = inverse_pow2(R3) * (P::kSplit ? kUntruncate / kPiScale : 1.f / kPiScale) + a.tab[2];
+        const float un = inverse_pow2(R3) * static_cast<float>(P::kOutputUp / kPiScale) + a.tab[2];
 #pragma unroll 1
         for (int c = 0; c < D; c += 32) {
           uint32_t v[32];
