@@ -1028,35 +1028,42 @@ unsigned int prefill_timeouts() {
   return v;
 }
 
-// Times in us, as measured: this path 28 and 2.2 per token tile and round of CTAs (whose rows all see every token tile in
-// the worst case); the decode kernels 20 and pairs of query row and token over their rate.
-bool prefill_pays(int64_t segs, int64_t nq, int64_t kv_len, int d, int terms) {
-  const double rows = (d == 128 && terms == 2) ? kRowsT : 2.0 * kRowsT;
-  const double rounds = ceil(segs * ceil(nq / rows) / kNumSMs);
-  const double mine = 28.0 + 2.2 * rounds * ((kv_len + kTok - 1) / kTok);
-  const double rate = terms == 1 ? 180e3 : (d == 64 ? 16e3 : 7e3);      // pairs per us, all SMs busy
-  const double theirs = 20.0 + 0.5 * segs * nq * kv_len / rate;
+// Times in us, fitted to 310 measured pairs (1 to 64 segments, 64 to 8192 rows, 256 to 16384 tokens): this path has a
+// constant and a time per token tile and round of CTAs, of which a round behind the first sees what is visible on average;
+// the decode kernels a constant and a rate of pairs of query row and token, hidden ones included.  At none of
+// them the way taken is more than 15 % behind the other (before, with one time per tile for all widths and half of the
+// decode kernels' time: 300 instead of 180 us for 2 segments x 256 rows x 4096 tokens at d = 128, 4 bits, and 104
+// instead of 56 us for 64 segments x 256 rows x 256 tokens over records).
+bool prefill_pays(int64_t segs, int64_t nq, int q_len, int64_t kv_len, int d, int terms, bool causal) {
+  const bool records = terms == 1, wide = d == 128 && !records;
+  const double rounds = ceil(segs * ceil(nq / (wide ? 1.0 * kRowsT : 2.0 * kRowsT)) / kNumSMs);
+  const double seen = causal && rounds > 1 ? 1.0 - 0.5 * (q_len - 1) / kv_len : 1.0;
+  const double mine = (records ? 42.0 : 34.0) + (records ? 3.0 : (wide ? 4.6 : 3.5)) * rounds * seen * ((kv_len + kTok - 1) / kTok);
+  const double theirs = (records ? 48.3 : (wide ? 44.0 : 36.0)) + 1.0 * segs * nq * kv_len / (records ? 200e3 : (wide ? 17.5e3 : 39e3));
   return mine < theirs;
 }
 
 // Whether the call's form is covered, and (unless forced) whether it is the faster way.
-bool prefill_rows_ok(int B, int Hkv, int64_t nq, int64_t kv_len, int d, int terms) {
+bool prefill_rows_ok(int B, int Hkv, int64_t group, int q_len, int64_t kv_len, int d, int terms, bool causal) {
+  const int64_t nq = group * q_len;
   const char* e = getenv("QUASHKV_B200_PREFILL_TCGEN05");      // 0 / 1: never / wherever it can, for A/B checks
   if (e && e[0] == '0') return false;
   if (!((d == 64 || d == 128) && nq <= 128 * 65535 && B * static_cast<int64_t>(Hkv) < 65535)) return false;
   if (e && e[0] == '1') return nq >= 16;
-  return nq >= kPrefillRows && prefill_pays(B * static_cast<int64_t>(Hkv), nq, kv_len, d, terms);
+  return nq >= kPrefillRows && prefill_pays(B * static_cast<int64_t>(Hkv), nq, q_len, kv_len, d, terms, causal);
 }
 
 size_t prefill_workspace_bytes(int B, int Hq, int Hkv, int q_len, int64_t kv_len, int d) {
-  const int64_t nq = static_cast<int64_t>(Hq / (Hkv > 0 ? Hkv : 1)) * q_len;
-  if (!prefill_rows_ok(B, Hkv, nq, kv_len, d, 2) && !prefill_rows_ok(B, Hkv, nq, kv_len, d, 1)) return 0;
+  // (asked without the mask: a causal call is taken wherever one without is)
+  const int64_t group = Hq / (Hkv > 0 ? Hkv : 1);
+  if (!prefill_rows_ok(B, Hkv, group, q_len, kv_len, d, 2, true) && !prefill_rows_ok(B, Hkv, group, q_len, kv_len, d, 1, true))
+    return 0;
   const size_t two = image_bytes(B, Hkv, kv_len, d, 2), one = image_bytes(B, Hkv, kv_len, d, 1);
   return two <= kMaxImageBytes ? two : (d == 128 && one <= kMaxImageBytes ? one : 0);
 }
 
 bool prefill_ok(const AttnArgs& s, size_t workspace_bytes) {
-  if (!prefill_rows_ok(s.B, s.Hkv, static_cast<int64_t>(s.G) * s.q_len, s.kv_len, s.d, s.records ? 1 : 2)) return false;
+  if (!prefill_rows_ok(s.B, s.Hkv, s.G, s.q_len, s.kv_len, s.d, s.records ? 1 : 2, s.causal != 0)) return false;
   const size_t need = image_bytes(s.B, s.Hkv, s.kv_len, s.d, s.records ? 1 : 2);
   return need <= kMaxImageBytes && need <= workspace_bytes && (reinterpret_cast<uintptr_t>(s.out) & 15u) == 0;
 }

@@ -189,6 +189,31 @@ def test_paged_append_of_a_repeated_sequence_id(monkeypatch):
     assert len(calls) == 2
 
 
+def test_many_query_rows_take_the_faster_kernels(monkeypatch):
+    """The choice shows in the workspace: token images for the prefill kernels or none.  Points on both sides of the
+    line, well away from it, with the measured times (decode kernels / prefill kernels, us)."""
+    L = _lib.lib()
+    for (B, Hq, Hkv, q_len, kv_len, d), taken in [
+            ((1, 8, 2, 64, 4096, 128), False),           # planes 180 / 300, records 57 / 216
+            ((1, 8, 2, 64, 16384, 128), False),          # 540 / 1080
+            ((1, 32, 8, 16, 4096, 128), False),          # 178 / 310
+            ((1, 8, 2, 64, 4096, 64), False),            # 95 / 253
+            ((1, 32, 8, 512, 4096, 128), True),          # 3700 / 344, records 305 / 224
+            ((8, 256, 64, 64, 256, 128), True),
+            ((8, 32, 4, 1024, 1024, 64), True),          # 8600 / 385
+            ((1, 32, 8, 256, 1024, 64), True)]:          # 318 / 86
+        args = (B, Hq, Hkv, q_len, kv_len, d)
+        monkeypatch.delenv("QUASHKV_B200_PREFILL_TCGEN05", raising=False)
+        auto = L.qkv_attention_workspace_bytes(*args)
+        monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "0")
+        decode = L.qkv_attention_workspace_bytes(*args)
+        monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "1")
+        prefill = L.qkv_attention_workspace_bytes(*args)
+        assert auto == (prefill if taken else decode), args
+        if prefill > decode:
+            assert (auto > decode) == taken, args
+
+
 def test_index_file_checks_without_gpu(tmp_path):
     """An empty index round-trips on CPU; foreign or inconsistent files are refused."""
     qk.QuashIndex(64, 4, seed=7).save(tmp_path / "empty.pt")
