@@ -165,12 +165,11 @@ std::tuple<Tensor, Tensor> compress_mixed(const Tensor& x_in, const Tensor& Pi_i
 
 struct AppendConsts { Tensor Pi, kb, kc, S, vb; };
 
-// (B, H, T, d) keys and values into the destination: one C call.
-void run_append(const Tensor& keys, const Tensor& values, const AppendConsts& c, int64_t mse_bits, int64_t val_bits,
-                const qkv_kv_dest_t& dest, void* stream) {
-  TORCH_CHECK_VALUE(keys.dim() == 4 && keys.sizes() == values.sizes(), "quashkv_b200: keys and values of shape (B, H, S, d)");
+// B * H segments of T new keys and values each into the destination: one C call.
+void run_append(const Tensor& keys, const Tensor& values, int64_t B, int64_t H, int64_t T, const AppendConsts& c,
+                int64_t mse_bits, int64_t val_bits, const qkv_kv_dest_t& dest, void* stream) {
   const at::Device dev = keys.device();
-  const int64_t B = keys.size(0), H = keys.size(1), T = keys.size(2), d = keys.size(3);
+  const int64_t d = keys.size(-1);
   const int64_t need = api.qkv_append_workspace_bytes(B, H, T, d, mse_bits, val_bits, dest.records != nullptr,
                                                       dest.block_table != nullptr);
   const Tensor ws = need > 0 ? empty({need}, at::kByte, dev) : Tensor();
@@ -180,19 +179,37 @@ void run_append(const Tensor& keys, const Tensor& values, const AppendConsts& c,
                           need > 0 ? ws.data_ptr() : nullptr, need, stream), "append");
 }
 
-// Row-major planes [B*H, capacity, ...], rows offset .. offset + S of every segment.
-void append_kv(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi, const Tensor& kb, const Tensor& kc,
-               const Tensor& S, int64_t mse_bits, const Tensor& vb, int64_t val_bits, Tensor k_codes, Tensor k_signs,
+// Row-major planes [segments, capacity, ...], rows offset .. offset + T of every segment: keys and values (..., T, d),
+// their leading dimensions flattened.  One C call where their shapes agree, else one for each.
+void append_kv(const Tensor& keys_in, const Tensor& values_in, const Tensor& Pi_in, const Tensor& kb_in, const Tensor& kc_in,
+               const Tensor& S_in, int64_t mse_bits, const Tensor& vb_in, int64_t val_bits, Tensor k_codes, Tensor k_signs,
                Tensor k_norms, Tensor v_codes, Tensor v_norms, int64_t offset) {
   const Tensor keys = data(keys_in), values = data(values_in);
   const at::Device dev = keys.device();
   Call call(dev);
   same_device(dev, {&values, &k_codes, &k_signs, &k_norms, &v_codes, &v_norms});
-  qkv_kv_dest_t dest{};
-  dest.k_codes = bpm(k_codes); dest.k_signs = bpm(k_signs); dest.k_norms = fpm(k_norms);
-  dest.v_codes = bpm(v_codes); dest.v_norms = fpm(v_norms);
-  dest.capacity = k_norms.size(-1); dest.offset = offset;
-  run_append(keys, values, {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
+  const int64_t T = keys.size(-2), d = keys.size(-1);
+  TORCH_CHECK_VALUE(values.size(-1) == d, "quashkv_b200: keys and values of different vector lengths");
+  if (keys.sizes() == values.sizes()) {
+    qkv_kv_dest_t dest{};
+    dest.k_codes = bpm(k_codes); dest.k_signs = bpm(k_signs); dest.k_norms = fpm(k_norms);
+    dest.v_codes = bpm(v_codes); dest.v_norms = fpm(v_norms);
+    dest.capacity = k_norms.size(-1); dest.offset = offset;
+    const bool four = keys.dim() == 4;
+    const int64_t B = four ? keys.size(0) : 1, H = four ? keys.size(1) : (keys.numel() > 0 ? keys.numel() / (T * d) : 0);
+    run_append(keys, values, B, H, T, {Pi_in, kb_in, kc_in, S_in, vb_in}, mse_bits, val_bits, dest, call.stream);
+    return;
+  }
+  const qkv_rows_t rows{T, k_norms.size(-1), offset};
+  const Tensor Pi = f32(Pi_in, dev), kb = f32(kb_in, dev), kc = f32(kc_in, dev), S = f32(S_in, dev), vb = f32(vb_in, dev);
+  check(api.qkv_compress_ip(keys.const_data_ptr(), dtype_code(keys), d, d > 0 ? keys.numel() / d : 0, d, fp(Pi), fp(kb), fp(kc),
+                            mse_bits, fp(S), bpm(k_codes), bpm(k_signs), 1, fpm(k_norms), rows, call.stream), "append keys");
+  check(api.qkv_compress_mse(values.const_data_ptr(), dtype_code(values), d, d > 0 ? values.numel() / d : 0, d, fp(Pi), fp(vb),
+                             val_bits, bpm(v_codes), 1, fpm(v_norms), rows, call.stream), "append values");
+}
+
+void check_bhtd(const Tensor& keys, const Tensor& values) {
+  TORCH_CHECK_VALUE(keys.dim() == 4 && keys.sizes() == values.sizes(), "quashkv_b200: keys and values of shape (B, H, T, d)");
 }
 
 // Tile records [B*H, capacity / 16, 1664], tokens offset .. offset + S of every segment.
@@ -206,7 +223,8 @@ void append_records(const Tensor& keys_in, const Tensor& values_in, const Tensor
   qkv_kv_dest_t dest{};
   dest.records = bpm(records);
   dest.capacity = capacity; dest.offset = offset;
-  run_append(keys, values, {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
+  check_bhtd(keys, values);
+  run_append(keys, values, keys.size(0), keys.size(1), keys.size(2), {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
 }
 
 // A pool of pages: planes = {records} or the five planes, positions start_lens[b] .. of the pages in block_table.
@@ -232,7 +250,8 @@ void append_paged(const Tensor& keys_in, const Tensor& values_in, const Tensor& 
   dest.start_lens = static_cast<const int32_t*>(lens.const_data_ptr());
   dest.max_blocks = static_cast<int>(table.size(1));
   dest.block_size = static_cast<int>(block_size);
-  run_append(keys, values, {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
+  check_bhtd(keys, values);
+  run_append(keys, values, keys.size(0), keys.size(1), keys.size(2), {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
 }
 
 // ---- decompress ---------------------------------------------------------------------------------------------------

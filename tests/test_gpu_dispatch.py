@@ -205,3 +205,30 @@ def test_prefill_over_records_is_no_further_from_64_bits_than_the_decode_kernels
             total[way] += float(row_errors(eng.attention(q, causal=causal), exact).square().mean())
     print(f"[precision] records: decode kernels {(total[0] / 6) ** 0.5:.3e}, prefill {(total[1] / 6) ** 0.5:.3e}")
     assert total[1] <= total[0] * 1.02 ** 2
+
+
+@pytest.mark.parametrize("lead", [(), (6,), (2, 3), (1, 2, 1, 3)])
+@pytest.mark.parametrize("D", [128, 64])
+def test_append_op_takes_any_leading_shape(lead, D):
+    """Keys and values (..., T, d) go to the planes' segments in the order of their flattened leading dimensions; values
+    of another leading shape (or fewer of them) to theirs."""
+    T, cap, off = 5, 24, 3
+    kq, vq = qk.InnerProductQuantizer(D, 3, seed=42, device=DEV), qk.MSEQuantizer(D, 3, seed=42, device=DEV)
+    Pi, kb, kc, S = kq._on(torch.device(DEV, 0))
+    vb = vq._on(torch.device(DEV, 0))[1]
+    g = torch.Generator(device=DEV).manual_seed(D)
+    segs = 1
+    for n in lead:
+        segs *= n
+    k, v = (torch.randn(*lead, T, D, generator=g, device=DEV) for _ in range(2))
+    codes, signs, norms = kq.compress_packed(k.reshape(segs, T, D))
+    v_codes, v_norms = vq.compress_packed(v.reshape(segs, T, D))
+    for values in (v, v.reshape(segs, T, D)[:1]):
+        planes = [torch.zeros(segs, cap, t.shape[-1], dtype=torch.uint8, device=DEV) for t in (codes, signs, v_codes)]
+        kn, vn = torch.zeros(segs, cap, device=DEV), torch.zeros(segs, cap, device=DEV)
+        qk.ops.append_kv(k, values, Pi, kb, kc, S, 2, vb, 3, planes[0], planes[1], kn, planes[2], vn, off)
+        n_v = values.numel() // (T * D)
+        for got, want, n in ((planes[0], codes, segs), (planes[1], signs, segs), (kn, norms, segs), (planes[2], v_codes, n_v),
+                             (vn, v_norms, n_v)):
+            assert torch.equal(got[:n, off:off + T], want[:n])
+            assert not got[:, :off].any() and not got[:, off + T:].any() and not got[n:].any()
