@@ -237,6 +237,10 @@ void append_paged(const Tensor& keys_in, const Tensor& values_in, const Tensor& 
   for (const Tensor& p : planes) same_device(dev, {&p});
   same_device(dev, {&values, &table_in, &lens_in});
   const auto int32 = [](const Tensor& t) { return t.scalar_type() == at::kInt ? t.contiguous() : t.to(at::kInt).contiguous(); };
+  check_bhtd(keys, values);
+  TORCH_CHECK_VALUE(table_in.dim() == 2 && table_in.size(0) == keys.size(0) && lens_in.numel() == keys.size(0),
+                    "quashkv_b200: a block table and start lengths for ", keys.size(0), " sequences, got ", table_in.sizes(),
+                    " and ", lens_in.sizes());
   const Tensor table = int32(table_in), lens = int32(lens_in);
   qkv_kv_dest_t dest{};
   if (planes.size() == 1) {
@@ -250,7 +254,6 @@ void append_paged(const Tensor& keys_in, const Tensor& values_in, const Tensor& 
   dest.start_lens = static_cast<const int32_t*>(lens.const_data_ptr());
   dest.max_blocks = static_cast<int>(table.size(1));
   dest.block_size = static_cast<int>(block_size);
-  check_bhtd(keys, values);
   run_append(keys, values, keys.size(0), keys.size(1), keys.size(2), {Pi, kb, kc, S, vb}, mse_bits, val_bits, dest, call.stream);
 }
 

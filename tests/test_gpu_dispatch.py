@@ -232,3 +232,15 @@ def test_append_op_takes_any_leading_shape(lead, D):
                              (vn, v_norms, n_v)):
             assert torch.equal(got[:n, off:off + T], want[:n])
             assert not got[:, :off].any() and not got[:, off + T:].any() and not got[n:].any()
+
+
+def test_paged_append_op_refuses_tables_of_another_batch():
+    """The kernel reads a table row and a start per sequence: fewer of them are refused on the host."""
+    pool = QuashKVPagedCache(8, 2, 64, QuashKVPageConfig(block_size=16), device=DEV)
+    x = torch.zeros(3, 2, 1, 64, device=DEV)
+    table = torch.arange(6, dtype=torch.int32, device=DEV).reshape(3, 2)
+    starts = torch.zeros(3, dtype=torch.int32, device=DEV)
+    for t, s in ((table[:2], starts), (table, starts[:2]), (table[0], starts)):
+        with pytest.raises(ValueError, match="block table and start lengths for 3 sequences"):
+            pool._store(x, x, t, s)
+    pool._store(x, x, table, starts)
