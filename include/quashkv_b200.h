@@ -255,8 +255,9 @@ int qkv_scatter_rows(const void* src, void* dst, const int64_t* slots, int64_t n
  *                 contiguous (block_table == NULL): token t of segment b * H + h goes to row
  *                 (b * H + h) * capacity + offset + t;
  *                 paged: to position start_lens[b] + t of the pages block_table[b][..], rows of
- *                 (block * H + h) * block_size + position % block_size; a position outside the table is
- *                 dropped.
+ *                 (block * H + h) * block_size + position % block_size; a position outside the table
+ *                 (or in a block with a negative number) is dropped and counted
+ *                 (qkv_dropped_append_rows).
  *   workspace     qkv_append_workspace_bytes(...) bytes, 256-byte aligned (0 for small appends: they are
  *                 one launch that writes the cache directly). */
 typedef struct {
@@ -279,6 +280,10 @@ int qkv_append_kv(const void* keys, int k_dtype, const void* values, int v_dtype
                   const float* Pi, const float* k_boundaries, const float* k_centroids, const float* S, int mse_bits,
                   const float* v_boundaries, int val_bits, qkv_kv_dest_t dest,
                   void* workspace, size_t workspace_bytes, void* stream);
+
+/* Rows (one per token and head) that paged appends on the current device have dropped since the library was
+ * loaded.  Waits for the device; a diagnostic for a serving loop that keeps its own tables. */
+int64_t qkv_dropped_append_rows(void);
 
 /* ---- tile records: the cache layout of the fast decode path -----------------------------------------
  * For head_dim 128 with 3-bit keys (2-bit codes + sign bit) and 3-bit values the cache can be kept as

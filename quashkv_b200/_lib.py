@@ -78,6 +78,7 @@ SIGNATURES = {
                                  _i, _vp, _vp, _sz, _vp]),
     "qkv_append_workspace_bytes": (_sz, [_i, _i, _i64, _i, _i, _i, _i, _i]),
     "qkv_append_kv": (_i, [_vp, _i, _vp, _i, _i, _i, _i64, _i, _vp, _vp, _vp, _vp, _i, _vp, _i, KvDest, _vp, _sz, _vp]),
+    "qkv_dropped_append_rows": (_i64, []),
     "qkv_scatter_rows": (_i, [_vp, _vp, _vp, _i64, _i, _vp]),
     "qkv_index_workspace_bytes": (_sz, [_i64, _i, _i, _i]),
     "qkv_index_scan_topk": (_i, [_vp, _i, _i, _vp, _vp, _vp, _i64, _i, _vp, _vp, _vp, _f, _i, _i64, _vp, _vp,

@@ -12,11 +12,16 @@
 namespace qkv {
 namespace {
 
+__device__ unsigned long long g_slots_dropped = 0;        // rows without a slot, large paged appends
+
 __global__ void __launch_bounds__(256) slots_kernel(const int32_t* __restrict__ block_table,
                                                     const int32_t* __restrict__ start_lens, int max_blocks, int block_size,
                                                     int heads, int tokens, int64_t n, int64_t* __restrict__ slots) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) slots[i] = paged_row(block_table, start_lens, max_blocks, block_size, heads, tokens, i);
+  if (i >= n) return;
+  const int64_t slot = paged_row(block_table, start_lens, max_blocks, block_size, heads, tokens, i);
+  slots[i] = slot;
+  if (slot < 0) atomicAdd(&g_slots_dropped, 1ull);
 }
 
 size_t up(size_t b) { return (b + 255) / 256 * 256; }
@@ -43,6 +48,12 @@ bool large(int64_t n, int d) { return d == kMaxD && n >= kAppendTensorCore; }
 }  // namespace qkv
 
 using namespace qkv;
+
+extern "C" int64_t qkv_dropped_append_rows(void) {
+  unsigned long long v = 0;
+  cudaMemcpyFromSymbol(&v, g_slots_dropped, sizeof(v));
+  return static_cast<int64_t>(v + chain_rows_dropped());
+}
 
 extern "C" size_t qkv_append_workspace_bytes(int B, int H, int64_t tokens, int d, int mse_bits, int val_bits, int tiled,
                                              int paged) {

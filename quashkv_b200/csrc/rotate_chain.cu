@@ -25,6 +25,8 @@ namespace qkv {
 
 namespace {
 
+__device__ unsigned long long g_rows_dropped = 0;        // rows without a slot, small paged appends
+
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kCtasPerSm = 3;                  // 168 registers a thread; 68 KB of shared memory
@@ -303,6 +305,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) compress_small_kernel(Ch
         const int64_t n = v0 + v;
         const int64_t row = n < a.n_vec ? chain_row(args, a, n) : -1;
         row_s[v] = row;
+        if (row < 0 && n < a.n_vec && !second) atomicAdd(&g_rows_dropped, 1ull);
         if (row >= 0) {
           if (args.records) {
             float* nd = reinterpret_cast<float*>(args.records + (row >> 4) * tile::kBytes +
@@ -741,6 +744,12 @@ int launch_decompress_t(const DecompressArgs& a, cudaStream_t st) {
 }
 
 }  // namespace
+
+unsigned long long chain_rows_dropped() {
+  unsigned long long v = 0;
+  cudaMemcpyFromSymbol(&v, g_rows_dropped, sizeof(v));
+  return v;
+}
 
 int launch_compress_chain(ChainArgs& args, cudaStream_t st) {
   switch ((args.d + 31) / 32) {

@@ -81,6 +81,7 @@ struct DecompressArgs {
 // fp32 FMA chains on the CUDA cores (rotate_chain.cu): any dimension up to 128, any width and layout.
 int launch_compress_chain(ChainArgs& args, cudaStream_t st);
 int launch_decompress_chain(const DecompressArgs& a, cudaStream_t st);
+unsigned long long chain_rows_dropped();              // rows of paged appends that had no slot (device-wide counter)
 bool compress_prefers_chain(const CompressArgs& a);   // rotate_quant.cu: the dispatch rule
 // tcgen05 rotation (rotate_umma.cu, decompress_umma.cu): d == 128, packed rows.
 bool compress_umma_ok(const CompressArgs& a);

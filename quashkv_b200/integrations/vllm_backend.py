@@ -27,7 +27,7 @@ from typing import Optional, Sequence
 import numpy as np
 import torch
 
-from .. import ops
+from .. import _lib, ops
 from ..engine import QuashKVEngine
 from ..triton_kernels.attention import CompressedBlock
 
@@ -252,7 +252,8 @@ class QuashKVPagedCache:
         max_blocks) int32 and ``start_lens`` (n_seq) int32 live on the device, the new tokens of sequence i go to
         positions start_lens[i] .. start_lens[i] + new_tokens - 1 of its pages.  The slots are computed on the
         device: no host loop and no host-to-device copy per decode step.  The pool's own bookkeeping
-        (``seq_len``, ``free``) is not involved."""
+        (``seq_len``, ``free``) is not involved.  The host does not see the positions: a token whose position lies
+        outside its row of the table is not stored, and counted (``dropped_rows``)."""
         ops._need_cuda(keys, "QuashKVPagedCache.append_with_tables")
         n, H, T, D = keys.shape
         if H != self.num_kv_heads or D != self.head_size or values.shape != keys.shape or \
@@ -262,6 +263,12 @@ class QuashKVPagedCache:
         if T == 0:
             return
         self._store(keys, values, block_table, start_lens)
+
+    @staticmethod
+    def dropped_rows() -> int:
+        """Rows (one per token and head) that paged appends on the current device could not store because their
+        position was outside the block table.  Waits for the device."""
+        return int(_lib.lib().qkv_dropped_append_rows())
 
     def _store(self, keys: torch.Tensor, values: torch.Tensor, table: torch.Tensor, starts: torch.Tensor) -> None:
         """Compress (n_seq, heads, T, d) keys and values and file every token at its slot

@@ -244,3 +244,30 @@ def test_paged_append_op_refuses_tables_of_another_batch():
         with pytest.raises(ValueError, match="block table and start lengths for 3 sequences"):
             pool._store(x, x, t, s)
     pool._store(x, x, table, starts)
+
+
+@pytest.mark.parametrize("D,block", [(128, 16), (128, 12), (64, 16)])
+@pytest.mark.parametrize("n_seq,T", [(3, 40), (8, 800)])
+def test_positions_outside_the_table_are_dropped_and_counted(D, block, n_seq, T):
+    """Both kinds of append (one launch; through the tensor-core kernels from 6144 rows on at d = 128): tokens past the
+    table of their sequence store nothing, the count says how many, the others are where they belong."""
+    H, width = 2, 2 * (T // block // 2) - 1                    # a table that is too short for every sequence
+    room = width * block
+    pool = QuashKVPagedCache(n_seq * width + 1, H, D, QuashKVPageConfig(block_size=block), device=DEV)
+    ref = QuashKVPagedCache(n_seq * width + 1, H, D, QuashKVPageConfig(block_size=block), device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    k, v = (torch.randn(n_seq, H, T, D, generator=g, device=DEV) for _ in range(2))
+    table = torch.randperm(n_seq * width, generator=g, device=DEV).to(torch.int32).reshape(n_seq, width)
+    starts = torch.arange(n_seq, dtype=torch.int32, device=DEV) * 3
+    before = pool.dropped_rows()
+    pool.append_with_tables(k, v, table, starts)
+    lost = sum(max(0, 3 * i + T - room) for i in range(n_seq))
+    assert lost > 0 and pool.dropped_rows() - before == lost * H
+    for i in range(n_seq):                                     # what fits, in calls of one sequence and a few tokens
+        for t in range(0, room - 3 * i, 100):
+            m = min(100, room - 3 * i - t)
+            ref.append_with_tables(k[i:i + 1, :, t:t + m].contiguous(), v[i:i + 1, :, t:t + m].contiguous(), table[i:i + 1],
+                                   starts[i:i + 1] + t)
+    for name, plane in pool.planes.items():
+        assert torch.equal(plane, ref.planes[name]), name
+    assert pool.dropped_rows() - before == lost * H
