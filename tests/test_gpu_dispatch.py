@@ -101,41 +101,6 @@ def test_paged_append_of_a_repeated_sequence_id(D, block):
         assert all(torch.equal(t, want[name]) for name, t in one.rows_of(s).items())
 
 
-@pytest.mark.parametrize("D,bits,paged", [(64, 3, False), (128, 4, False), (128, 3, False), (64, 3, True), (128, 3, True)])
-def test_prefill_rows_are_right_after_a_wait_that_ran_out(D, bits, paged, monkeypatch):
-    """One token tile of the first CTA is never multiplied: its bounded waits run out, are counted, and its rows come
-    from the fp32 way out, while the rows of the other CTAs stay what they are.  (d = 128 at 3/3 bits: both kernels
-    beside it round to fp16, the way out does not.)"""
-    n, q_len, G = 200, 100, 4
-    g = torch.Generator(device=DEV).manual_seed(D + bits)
-    k, v = (_outliers(g, (2, 1, n, D), torch.bfloat16) for _ in range(2))
-    q = torch.randn(2, G, q_len, D, generator=g, device=DEV)
-    if paged:
-        pool = QuashKVPagedCache(32, 1, D, QuashKVPageConfig(key_bits=bits, value_bits=bits, block_size=16), device=DEV)
-        pool.append(["a", "b"], k, v)
-        attend = lambda causal: pool.attention(["a", "b"], q, causal=causal)      # noqa: E731
-    else:
-        eng = qk.QuashKVEngine(D, bits, bits, seed=42, device=DEV, pack_storage=True)
-        eng.append(k, v)
-        attend = lambda causal: eng.attention(q, causal=causal)      # noqa: E731
-    bound = 1e-3 if (D, bits) == (128, 3) else 5e-6
-    for causal in (False, True):
-        monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "0")
-        want = attend(causal)
-        monkeypatch.setenv("QUASHKV_B200_PREFILL_TCGEN05", "1")
-        count = _lib.lib().qkv_tensor_core_timeouts()
-        plain = attend(causal)
-        assert _lib.lib().qkv_tensor_core_timeouts() == count
-        monkeypatch.setenv("QUASHKV_B200_TEST_DROP_MMA", "1")
-        torch.empty(1 << 20, device=DEV).fill_(float("nan"))      # what an unwritten output would likely show
-        got = attend(causal)
-        assert _lib.lib().qkv_tensor_core_timeouts() > count
-        monkeypatch.delenv("QUASHKV_B200_TEST_DROP_MMA")
-        assert rel_l2(got, want) < bound and rel_l2(got[0], want[0]) < bound
-        assert torch.equal(got[1], plain[1]) and not torch.equal(got[0], plain[0])
-        assert torch.equal(attend(causal), plain)
-
-
 @pytest.mark.parametrize("log2_step", [10, 20, 34, 60])
 @pytest.mark.parametrize("D,bits", [(64, 3), (64, 4), (128, 4), (128, 3)])
 def test_prefill_keeps_rows_beside_a_much_larger_value_norm(D, bits, log2_step, monkeypatch):
