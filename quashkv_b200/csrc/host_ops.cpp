@@ -12,6 +12,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/library.h>
 
 #include <tuple>
@@ -434,9 +436,52 @@ TORCH_LIBRARY_IMPL(quashkv_b200, CUDA, m) {
 #undef QKV_IMPL
 }
 
-// Compressed codes are not differentiable: the autograd keys are passed through (no graph, no boxed fallback).
+namespace {
+
+// Nothing here has a derivative: where gradients are wanted, the floating-point results carry a node that says so in the
+// backward pass instead of ending the graph without a word.  What the op calls itself records nothing.
+void without_derivative(const c10::OperatorHandle& op, c10::DispatchKeySet keys, torch::jit::Stack* stack) {
+  std::vector<Tensor> inputs;
+  if (c10::GradMode::is_enabled())
+    for (const c10::IValue& v : torch::jit::last(*stack, op.schema().arguments().size()))
+      if (v.isTensor() && v.toTensor().defined() && v.toTensor().requires_grad()) inputs.push_back(v.toTensor());
+  {
+    at::AutoDispatchBelowAutograd below;
+    op.redispatchBoxed(keys & c10::after_autograd_keyset, stack);
+  }
+  if (inputs.empty()) return;
+  const std::shared_ptr<torch::autograd::Node> node(new torch::autograd::NotImplemented(op.schema().name()),
+                                                    torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(inputs));
+  for (const c10::IValue& v : torch::jit::last(*stack, op.schema().returns().size()))
+    if (v.isTensor() && v.toTensor().is_floating_point()) torch::autograd::set_history(v.toTensor(), node);
+}
+
+// Tensors that the op writes count the write, so that a graph that saved one of them notices.
+void count_writes(const c10::OperatorHandle& op, c10::DispatchKeySet keys, torch::jit::Stack* stack) {
+  const auto bump = [](const Tensor& t) {
+    if (t.defined() && !t.is_inference()) t.unsafeGetTensorImpl()->bump_version();
+  };
+  const auto& args = op.schema().arguments();
+  const auto values = torch::jit::last(*stack, args.size());
+  for (size_t i = 0; i < args.size(); ++i) {
+    if (args[i].alias_info() == nullptr || !args[i].alias_info()->isWrite()) continue;
+    if (values[i].isTensor()) bump(values[i].toTensor());
+    if (values[i].isTensorList())
+      for (const Tensor& t : values[i].toTensorVector()) bump(t);
+  }
+  op.redispatchBoxed(keys & c10::after_ADInplaceOrView_keyset, stack);
+}
+
+}  // namespace
+
 TORCH_LIBRARY_IMPL(quashkv_b200, Autograd, m) {
-#define QKV_SKIP(name) m.impl(#name, torch::CppFunction::makeFallthrough());
-  QKV_FOR_EACH_OP(QKV_SKIP)
-#undef QKV_SKIP
+#define QKV_NO_DERIVATIVE(name) m.impl(#name, torch::CppFunction::makeFromBoxedFunction<&without_derivative>());
+  QKV_FOR_EACH_OP(QKV_NO_DERIVATIVE)
+#undef QKV_NO_DERIVATIVE
+}
+
+TORCH_LIBRARY_IMPL(quashkv_b200, ADInplaceOrView, m) {
+  for (const char* name : {"compress_ip_into", "append_kv", "append_records", "append_paged", "attention_tiled_out"})
+    m.impl(name, torch::CppFunction::makeFromBoxedFunction<&count_writes>());
 }

@@ -230,6 +230,7 @@ class QuashKVEngine:
         Pi, _, k_cents, Sgn = kq._on(queries.device)
         _, _, v_cents = vq._on(queries.device)
         p = self._planes
+        queries = queries.detach()               # (inference: the result is outside any graph)
         if self._tiled:
             return ops.attention_tiled(queries, p["records"], self._capacity, self._total_tokens, Hkv, None, None, 0, Pi,
                                        k_cents, v_cents, Sgn, kq.qjl_scale, float(scale), bool(causal))

@@ -236,3 +236,21 @@ def test_positions_outside_the_table_are_dropped_and_counted(D, block, n_seq, T)
     for name, plane in pool.planes.items():
         assert torch.equal(plane, ref.planes[name]), name
     assert pool.dropped_rows() - before == lost * H
+
+
+def test_a_backward_pass_through_an_op_is_refused():
+    """Gradients that do not exist are an error where they are asked for; the engine's attention is outside any graph."""
+    pool = QuashKVPagedCache(4, 2, 64, QuashKVPageConfig(block_size=16), device=DEV)
+    k = torch.randn(1, 2, 20, 64, device=DEV)
+    pool.append(["a"], k, k)
+    q = torch.randn(1, 4, 1, 64, device=DEV, requires_grad=True)
+    with pytest.raises(RuntimeError, match="not implemented"):
+        (pool.attention(["a"], q).sum() + q.sum()).backward()
+    eng = qk.QuashKVEngine(64, 3, 3, seed=42, device=DEV)
+    eng.append(k.requires_grad_(), k)
+    assert not eng.attention(q).requires_grad
+    with torch.no_grad():
+        assert torch.equal(eng.attention(q), eng.attention(q.detach()))
+    with torch.inference_mode():
+        eng.append(torch.randn(1, 2, 3, 64, device=DEV), torch.randn(1, 2, 3, 64, device=DEV))
+        assert eng.attention(torch.randn(1, 4, 1, 64, device=DEV)).shape == (1, 4, 1, 64)

@@ -214,6 +214,47 @@ def test_many_query_rows_take_the_faster_kernels(monkeypatch):
             assert (auto > decode) == taken, args
 
 
+def _fake_calls():
+    """Arguments of the ops over d = 128 planes, as fake CUDA tensors (call inside a FakeTensorMode)."""
+    u8 = lambda *s: torch.empty(*s, dtype=torch.uint8, device="cuda")      # noqa: E731
+    f32 = lambda *s: torch.empty(*s, device="cuda")      # noqa: E731
+    consts = (f32(128, 128), f32(3), f32(4), f32(128), 2, f32(7), 3)
+    planes = [u8(2, 64, 32), u8(2, 64, 16), f32(2, 64), u8(2, 64, 48), f32(2, 64)]
+    tail = (f32(128, 128), f32(4), f32(8), f32(128), 0.1, 0.1, False)
+    return u8, f32, consts, planes, tail
+
+
+def test_results_of_differentiable_inputs_carry_a_node_and_written_tensors_count_it():
+    """Nothing here has a derivative: a result of inputs that want gradients must not leave the graph silently, and a
+    tensor that an op writes counts the write (no GPU: fake tensors pass the same dispatch keys)."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    _lib.load_host()
+    O = torch.ops.quashkv_b200
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        u8, f32, consts, planes, tail = _fake_calls()
+        x, q = f32(1, 2, 8, 128).requires_grad_(), f32(1, 2, 1, 128).requires_grad_()
+        records = u8(2, 4, 1664)
+        codes, norms = O.compress_mse(x, f32(128, 128), f32(7), 3, True)
+        assert not codes.requires_grad and norms.requires_grad
+        out = O.attention_tiled(q, records, 64, 8, 2, None, None, 0, *tail)
+        paged = O.attention_paged(q, *(p.reshape(4, 2, 16, -1) for p in planes), torch.empty(1, 4, dtype=torch.int32, device="cuda"),
+                                  torch.empty(1, dtype=torch.int32, device="cuda"), 8, 3, 3, *tail)
+        scores, ids = O.index_scan_topk(q.reshape(2, 128), *planes[:3], 64, 2, *tail[:1], f32(4), f32(128), 0.1, 4, 0)
+        assert out.requires_grad and paged.requires_grad and scores.requires_grad and not ids.requires_grad
+        with torch.no_grad():
+            assert not O.attention_tiled(q, records, 64, 8, 2, None, None, 0, *tail).requires_grad
+        assert not O.attention_tiled(q.detach(), records, 64, 8, 2, None, None, 0, *tail).requires_grad
+        O.append_kv(x, x, *consts, *planes, 0)
+        O.append_records(x, x, *consts, records, 64, 0)
+        O.append_paged(x, x, *consts, planes, torch.empty(1, 4, dtype=torch.int32, device="cuda"),
+                       torch.empty(1, dtype=torch.int32, device="cuda"), 16)
+        O.compress_ip_into(x, *consts[:5], *planes[:3], 0)
+        written = f32(1, 2, 1, 128)
+        O.attention_tiled_out(q, records, 64, 8, 2, None, None, 0, *tail, written)
+        assert [p._version for p in planes] == [3, 3, 3, 2, 2] and records._version == 1 and written._version == 1
+        assert x._version == 0 and not any(t.requires_grad for t in (*planes, records, written))
+
+
 def test_index_file_checks_without_gpu(tmp_path):
     """An empty index round-trips on CPU; foreign or inconsistent files are refused."""
     qk.QuashIndex(64, 4, seed=7).save(tmp_path / "empty.pt")
