@@ -89,38 +89,38 @@ class _Keep:
 # Ops implemented in csrc/host_ops.cpp.
 _LIBRARY = torch.library.Library("quashkv_b200", "FRAGMENT")
 _CONSTS = "Tensor Pi, Tensor key_centroids, Tensor val_centroids, Tensor S, float qjl_scale, float scale, bool causal"
-_APPEND = ("Tensor keys, Tensor values, Tensor Pi, Tensor k_bounds, Tensor k_cents, Tensor S, int mse_bits, "
-           "Tensor v_bounds, int val_bits")
-_TILED = ("Tensor q, Tensor records, int capacity, int kv_len, int n_kv_heads, Tensor? block_table, Tensor? seq_lens, "
-          f"int block_size, {_CONSTS}")
+_APPEND = ("Tensor keys, Tensor values, Tensor Pi, Tensor k_bounds, Tensor k_cents, Tensor S, SymInt mse_bits, "
+           "Tensor v_bounds, SymInt val_bits")
+_TILED = ("Tensor q, Tensor records, SymInt capacity, SymInt kv_len, SymInt n_kv_heads, Tensor? block_table, Tensor? seq_lens, "
+          f"SymInt block_size, {_CONSTS}")
 for _schema in (
-        "compress_mse(Tensor x, Tensor Pi, Tensor boundaries, int bits, bool packed) -> (Tensor, Tensor)",
-        "compress_ip(Tensor x, Tensor Pi, Tensor boundaries, Tensor centroids, Tensor S, int mse_bits, bool packed) "
+        "compress_mse(Tensor x, Tensor Pi, Tensor boundaries, SymInt bits, bool packed) -> (Tensor, Tensor)",
+        "compress_ip(Tensor x, Tensor Pi, Tensor boundaries, Tensor centroids, Tensor S, SymInt mse_bits, bool packed) "
         "-> (Tensor, Tensor, Tensor)",
-        "compress_ip_into(Tensor x, Tensor Pi, Tensor boundaries, Tensor centroids, Tensor S, int mse_bits, "
-        "Tensor(a!) codes, Tensor(b!) signs, Tensor(c!) norms, int offset) -> ()",
-        "compress_mixed(Tensor x, Tensor Pi, Tensor is_outlier, Tensor bounds_out, int bits_out, Tensor bounds_reg, "
-        "int bits_reg, bool packed, int n_out) -> (Tensor, Tensor)",
+        "compress_ip_into(Tensor x, Tensor Pi, Tensor boundaries, Tensor centroids, Tensor S, SymInt mse_bits, "
+        "Tensor(a!) codes, Tensor(b!) signs, Tensor(c!) norms, SymInt offset) -> ()",
+        "compress_mixed(Tensor x, Tensor Pi, Tensor is_outlier, Tensor bounds_out, SymInt bits_out, Tensor bounds_reg, "
+        "SymInt bits_reg, bool packed, SymInt n_out) -> (Tensor, Tensor)",
         f"append_kv({_APPEND}, Tensor(a!) k_codes, Tensor(b!) k_signs, Tensor(c!) k_norms, Tensor(d!) v_codes, "
-        "Tensor(e!) v_norms, int offset) -> ()",
-        f"append_records({_APPEND}, Tensor(a!) records, int capacity, int offset) -> ()",
-        f"append_paged({_APPEND}, Tensor(a!)[] planes, Tensor block_table, Tensor start_lens, int block_size) -> ()",
-        "decompress(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, int bits, Tensor? S, "
-        "float qjl_scale, bool packed, int d, int seg_len, int seg_stride, int seg_off, int n_vec, "
+        "Tensor(e!) v_norms, SymInt offset) -> ()",
+        f"append_records({_APPEND}, Tensor(a!) records, SymInt capacity, SymInt offset) -> ()",
+        f"append_paged({_APPEND}, Tensor(a!)[] planes, Tensor block_table, Tensor start_lens, SymInt block_size) -> ()",
+        "decompress(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, SymInt bits, Tensor? S, "
+        "float qjl_scale, bool packed, SymInt d, SymInt seg_len, SymInt seg_stride, SymInt seg_off, SymInt n_vec, "
         "ScalarType out_dtype) -> Tensor",
-        "decompress_dense(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, int bits, Tensor? S, "
-        "float qjl_scale, bool packed, int d, ScalarType out_dtype) -> Tensor",
-        "decompress_mixed(Tensor codes, Tensor norms, Tensor Pi, Tensor is_outlier, Tensor cents_out, int bits_out, "
-        "Tensor cents_reg, int bits_reg, bool packed, int d) -> Tensor",
+        "decompress_dense(Tensor codes, Tensor? signs, Tensor norms, Tensor Pi, Tensor centroids, SymInt bits, Tensor? S, "
+        "float qjl_scale, bool packed, SymInt d, ScalarType out_dtype) -> Tensor",
+        "decompress_mixed(Tensor codes, Tensor norms, Tensor Pi, Tensor is_outlier, Tensor cents_out, SymInt bits_out, "
+        "Tensor cents_reg, SymInt bits_reg, bool packed, SymInt d) -> Tensor",
         "attention(Tensor q, Tensor k_codes, Tensor k_signs, Tensor k_norms, Tensor v_codes, Tensor v_norms, "
-        f"int kv_len, int n_kv_heads, int key_bits, int val_bits, {_CONSTS}) -> Tensor",
+        f"SymInt kv_len, SymInt n_kv_heads, SymInt key_bits, SymInt val_bits, {_CONSTS}) -> Tensor",
         "attention_paged(Tensor q, Tensor k_codes, Tensor k_signs, Tensor k_norms, Tensor v_codes, Tensor v_norms, "
-        f"Tensor block_table, Tensor seq_lens, int max_kv_len, int key_bits, int val_bits, {_CONSTS}) -> Tensor",
+        f"Tensor block_table, Tensor seq_lens, SymInt max_kv_len, SymInt key_bits, SymInt val_bits, {_CONSTS}) -> Tensor",
         f"attention_tiled({_TILED}) -> Tensor",
         f"attention_tiled_out({_TILED}, Tensor(a!) out) -> ()",
-        "index_scan_topk(Tensor queries, Tensor db_codes, Tensor db_signs, Tensor db_norms, int n_vectors, int bits, "
-        "Tensor Pi, Tensor centroids, Tensor S, float qjl_scale, int k, int id_base) -> (Tensor, Tensor)"):
-    _LIBRARY.define(_schema)
+        "index_scan_topk(Tensor queries, Tensor db_codes, Tensor db_signs, Tensor db_norms, SymInt n_vectors, SymInt bits, "
+        "Tensor Pi, Tensor centroids, Tensor S, float qjl_scale, SymInt k, SymInt id_base) -> (Tensor, Tensor)"):
+    _LIBRARY.define(_schema, tags=torch.Tag.pt2_compliant_tag)
 _NATIVE = torch.ops.quashkv_b200
 _lib.load_host(required=False)        # not built yet: the first call says so
 

@@ -255,6 +255,28 @@ def test_results_of_differentiable_inputs_carry_a_node_and_written_tensors_count
         assert x._version == 0 and not any(t.requires_grad for t in (*planes, records, written))
 
 
+def test_native_ops_are_traced_with_symbolic_sizes():
+    """Lengths and offsets that change from call to call (kv_len, offset, n_vectors) stay symbols under tracing: one
+    graph for all of them."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.symbolic_shapes import ShapeEnv
+    _lib.load_host()
+    O, env = torch.ops.quashkv_b200, ShapeEnv()
+    with FakeTensorMode(allow_non_fake_inputs=True, shape_env=env):
+        u8, f32, consts, planes, tail = _fake_calls()
+        n, x = env.create_unbacked_symint(), f32(1, 2, 8, 128)
+        O.append_kv(x, x, *consts, *planes, n)
+        O.append_records(x, x, *consts, u8(2, 4, 1664), n, n)
+        O.compress_ip_into(x, *consts[:5], *planes[:3], n)
+        out = O.attention_tiled(f32(1, 2, 1, 128), u8(2, 4, 1664), n, n, 2, None, None, 0, *tail)
+        O.attention(f32(1, 2, 1, 128), *planes, n, 2, 3, 3, *tail)
+        O.index_scan_topk(f32(2, 128), *planes[:3], n, 2, *tail[:1], f32(4), f32(128), 0.1, 4, n)
+        rows = O.decompress(planes[0], None, planes[2], f32(128, 128), f32(4), 2, None, 0.0, True, 128, 8, n, n, 16, torch.float32)
+    assert out.shape == (1, 2, 1, 128) and rows.shape == (16, 128)
+    for name in ("compress_mse", "append_paged", "attention", "attention_paged", "attention_tiled", "index_scan_topk"):
+        assert torch.Tag.pt2_compliant_tag in getattr(O, name).default.tags
+
+
 def test_index_file_checks_without_gpu(tmp_path):
     """An empty index round-trips on CPU; foreign or inconsistent files are refused."""
     qk.QuashIndex(64, 4, seed=7).save(tmp_path / "empty.pt")
