@@ -8,6 +8,7 @@ the hot ops over torch's C++ API).
 from __future__ import annotations
 
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -46,13 +47,31 @@ def _stale() -> bool:
     return _newer(LIB_PATH, _sources() + _headers())
 
 
-def _build_host() -> None:
-    """The ops' host side, against the headers of the torch that is installed (found without importing it)."""
+def _torch_dir() -> str:
+    """Where the installed torch is, without importing it."""
     from importlib.util import find_spec
-    torch_dir = os.path.dirname(find_spec("torch").origin)
+    return os.path.dirname(find_spec("torch").origin)
+
+
+def _host_mark() -> str:
+    """What the host library says of itself: the torch whose C++ interface it was compiled against."""
+    with open(os.path.join(_torch_dir(), "version.py")) as f:
+        version = re.search(r"__version__ = '([^']+)'", f.read()).group(1)
+    return f"quashkv_host for torch {version};"
+
+
+def host_fits_torch() -> bool:
+    """Whether the built host library belongs to the torch that is installed (another one's C++ interface may differ)."""
+    with open(HOST_PATH, "rb") as f:
+        return _host_mark().encode() in f.read()
+
+
+def _build_host() -> None:
+    """The ops' host side, against the headers of the torch that is installed."""
+    torch_dir = _torch_dir()
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     cuda_dir = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{torch_dir}/include",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f'-DQKV_HOST_MARK="{_host_mark()}"', f"-I{torch_dir}/include",
            f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{cuda_dir}/include", HOST_SOURCE, "-o", HOST_PATH + ".new",
            f"-L{torch_dir}/lib", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
@@ -65,7 +84,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     """Compile the CUDA sources when the library is missing or older than a source.  Every source becomes an
     object file of its own (compiled side by side, kept under lib/obj so that a change rebuilds one file),
     then the objects are linked into the shared library."""
-    if force or _newer(HOST_PATH, [HOST_SOURCE] + _headers()[-1:]):
+    if force or _newer(HOST_PATH, [HOST_SOURCE] + _headers()[-1:]) or not host_fits_torch():
         os.makedirs(LIB_DIR, exist_ok=True)
         _build_host()
     if not force and not _stale():

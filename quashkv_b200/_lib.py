@@ -10,7 +10,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from ._build import HOST_PATH, LIB_PATH
+from ._build import HOST_PATH, LIB_PATH, host_fits_torch
 
 F32, BF16, F16 = 0, 1, 2
 INDEX_MAX_K = 128
@@ -97,25 +97,36 @@ def _path() -> str:
 
 
 def load_host(required: bool = True) -> None:
-    """Register the native implementations of the hot ops (csrc/host_ops.cpp) and point them at the library."""
+    """Register the native implementations of the hot ops (csrc/host_ops.cpp) and point them at the library.
+
+    ``required=False`` (at import): libraries that are missing, stale or built against another torch are left alone,
+    since the build that replaces them imports the package too; the first call that needs them says what is wrong."""
     global HOST_READY
-    if HOST_READY or (not required and not (os.path.exists(HOST_PATH) and os.path.exists(_path()))):
+    if HOST_READY:
         return
     try:
-        lib()
-    except AttributeError:       # a library older than this file: the build that replaces it imports the package too
+        _load_host()
+    except Exception:
         if required:
             raise
         return
+    HOST_READY = True
+
+
+def _load_host() -> None:
+    lib()
     if not os.path.exists(HOST_PATH):
         raise RuntimeError(
             f"quashkv_b200: {HOST_PATH} not found. Build it with `python -m quashkv_b200._build`; "
             "there is no fallback implementation.")
+    if not host_fits_torch():
+        raise RuntimeError(f"quashkv_b200: {HOST_PATH} was built against another torch; "
+                           "rebuild it with `python -m quashkv_b200._build`")
     import torch
     torch.ops.load_library(HOST_PATH)
     if C.CDLL(HOST_PATH).quashkv_host_bind(_path().encode()) != 0:
-        raise RuntimeError(f"quashkv_b200: {_path()} lacks an entry point that {HOST_PATH} calls; rebuild both")
-    HOST_READY = True
+        raise RuntimeError(f"quashkv_b200: {_path()} lacks an entry point that {HOST_PATH} calls; "
+                           "rebuild both with `python -m quashkv_b200._build`")
 
 
 def lib() -> C.CDLL:

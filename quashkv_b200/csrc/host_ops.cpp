@@ -35,6 +35,7 @@ struct Api {
   QKV_FOR_EACH_ENTRY(QKV_MEMBER)
 #undef QKV_MEMBER
 } api;
+bool bound = false;           // every entry point resolved
 
 void check(int rc, const char* what) {
   TORCH_CHECK(rc == 0, "quashkv_b200: ", what, " failed: ", api.qkv_strerror(rc), " (code ", rc, ")");
@@ -89,7 +90,9 @@ Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Device& dev) {
 struct Call {             // device guard and stream of one op
   c10::cuda::CUDAGuard guard;
   void* stream;
-  explicit Call(const at::Device& dev) : guard(dev), stream(c10::cuda::getCurrentCUDAStream(dev.index()).stream()) {}
+  explicit Call(const at::Device& dev) : guard(dev), stream(c10::cuda::getCurrentCUDAStream(dev.index()).stream()) {
+    TORCH_CHECK(bound, "quashkv_b200: the library has not been loaded; rebuild it with `python -m quashkv_b200._build`");
+  }
 };
 
 int64_t row_bytes(int64_t d, int64_t bits) {
@@ -416,6 +419,7 @@ std::tuple<Tensor, Tensor> index_scan_topk(const Tensor& q_in, const Tensor& cod
 
 // Resolves the entry points in the library at `path` (the one the Python side has loaded).  0, or 1 on failure.
 extern "C" int quashkv_host_bind(const char* path) {
+  bound = false;
   void* handle = dlopen(path, RTLD_NOW | RTLD_LOCAL);
   if (handle == nullptr) return 1;
 #define QKV_RESOLVE(name)                                                 \
@@ -423,8 +427,12 @@ extern "C" int quashkv_host_bind(const char* path) {
   if (api.name == nullptr) return 1;
   QKV_FOR_EACH_ENTRY(QKV_RESOLVE)
 #undef QKV_RESOLVE
+  bound = true;
   return 0;
 }
+
+// The torch that this file was compiled against, for the loader (which looks for it in the file before loading it).
+extern "C" __attribute__((used, visibility("default"))) const char quashkv_host_mark[] = QKV_HOST_MARK;
 
 #define QKV_FOR_EACH_OP(X)                                                                                          \
   X(compress_mse) X(compress_ip) X(compress_ip_into) X(compress_mixed) X(append_kv) X(append_records) X(append_paged) X(decompress) X(decompress_dense) \

@@ -451,3 +451,41 @@ def test_every_cuda_source_is_part_of_the_build():
     from quashkv_b200 import _build
     on_disk = sorted(f for f in os.listdir(_build.CSRC) if f.endswith(".cu"))
     assert sorted(_build.SOURCES) == on_disk
+
+
+@pytest.mark.parametrize("fault", ["no library at all", "another torch", "an older library"])
+def test_package_with_a_stale_host_library_imports_and_says_so(tmp_path, fault):
+    """The build imports the package: a host library that cannot be loaded must not stand in its way, and the first
+    call names it and the command that mends it."""
+    import shutil
+    import subprocess
+    import sys
+    from quashkv_b200 import _build
+    pkg = tmp_path / "quashkv_b200"
+    shutil.copytree(os.path.join(ROOT, "quashkv_b200"), pkg, ignore=shutil.ignore_patterns("lib", "__pycache__"))
+    shutil.copytree(os.path.join(ROOT, "include"), tmp_path / "include")
+    (pkg / "lib").mkdir()
+    os.symlink(_build.LIB_PATH, pkg / "lib" / "libquashkv_b200.so")
+    host = pkg / "lib" / "quashkv_host.so"
+    with open(_build.HOST_PATH, "rb") as f:
+        built = f.read()
+    mark = _build._host_mark().encode()
+    assert mark in built
+    if fault == "another torch":
+        host.write_bytes(built.replace(mark, b"x" * len(mark)))
+    elif fault == "an older library":            # one that calls an entry point which the library beside it lacks
+        host.write_bytes(built.replace(b"qkv_append_kv\0", b"qkv_append_kx\0"))
+    else:
+        host.write_bytes(b"not a library; " + mark)
+    code = ("import quashkv_b200, torch\n"
+            "from quashkv_b200 import _build, _lib\n"
+            "print('imported', _lib.HOST_READY)\n"
+            "try:\n    _lib.load_host()\nexcept Exception as e:\n    print('refused', e)\n"
+            f"print('stale', not _build.host_fits_torch())\n")
+    env = {k: v for k, v in os.environ.items() if not k.startswith("QUASHKV")}
+    run = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, env=env, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
+    assert "imported False" in run.stdout and "refused" in run.stdout
+    assert ("stale True" in run.stdout) == (fault == "another torch")
+    if fault != "no library at all":
+        assert "python -m quashkv_b200._build" in run.stdout
