@@ -12,11 +12,13 @@
 //   memory, a broadcast that still costs a return slot of 128 bytes a cycle, so this form runs at a quarter of the FMA
 //   rate: right for latency, wrong for bulk.
 // bulk (compress_bulk_kernel, decompress_bulk_kernel): a thread owns 8 coordinates x 8 vectors; both operands come from
-//   shared memory as float4, 64 FMAs per four loads, where FMA rate and load return balance.
+//   shared memory as float4, 64 FMAs per four loads, where FMA rate and load return balance.  Up to four CTAs share an
+//   SM, so that one loads while another multiplies: 400,000 vectors of 64 at 2 bits, compress fp32 300 (two CTAs) -> 211
+//   us, bf16 360 -> 198, decompress to fp32 285 -> 165.
 //
-// The keys and values of an append run as ONE launch (two jobs), and the small kernel writes their codes straight to
-// where the cache keeps them: row-major planes, or the tile records of the d = 128, 3/3-bit cache, contiguous or
-// through a block table.
+// The keys and values of an append run as ONE launch (two jobs), and both kernels write their codes straight to where the
+// cache keeps them: row-major planes, contiguous or through a block table; the small one also the tile records of the
+// d = 128, 3/3-bit cache.
 #include "mma_decode.cuh"
 #include "rotate_common.cuh"
 #include "tile_format.cuh"
@@ -174,15 +176,19 @@ template <int PER_LANE> struct ChannelFields {
       sgn[t] = (a.signs && j < d) ? a.S[j] : 0.f;
     }
   }
-  __device__ __forceinline__ float value(const DecompressArgs& a, const float (*tab)[16], int64_t row, int t, int lane) const {
+  __device__ __forceinline__ uint32_t code(const DecompressArgs& a, int64_t row, int t, int lane) const {
+    return a.packed ? read_field(a.codes + row * row_bytes, bitpos[t], width[t], row_bytes) : a.codes[row * a.d + lane + 32 * t];
+  }
+  __device__ __forceinline__ uint32_t sign(const DecompressArgs& a, int64_t row, int t, int lane) const {
     const int j = lane + 32 * t;
-    const uint32_t c = a.packed ? read_field(a.codes + row * row_bytes, bitpos[t], width[t], row_bytes) : a.codes[row * a.d + j];
-    float y = tab[cls[t]][c & 15u];
-    if (a.signs) {
-      const uint32_t sb = a.packed ? ((a.signs[row * sign_bytes + (j >> 3)] >> (j & 7)) & 1u) : a.signs[row * a.d + j];
-      y += a.qjl_scale * (sgn[t] * (sb ? 1.f : -1.f));
-    }
-    return y;
+    return a.packed ? ((a.signs[row * sign_bytes + (j >> 3)] >> (j & 7)) & 1u) : a.signs[row * a.d + j];
+  }
+  __device__ __forceinline__ float sign_term(const DecompressArgs& a, uint32_t sb, int t) const {
+    return a.qjl_scale * (sgn[t] * (sb ? 1.f : -1.f));
+  }
+  __device__ __forceinline__ float value(const DecompressArgs& a, const float (*tab)[16], int64_t row, int t, int lane) const {
+    const float y = tab[cls[t]][code(a, row, t, lane) & 15u];
+    return a.signs ? y + sign_term(a, sign(a, row, t, lane), t) : y;
   }
 };
 
@@ -448,6 +454,8 @@ template <int DR> struct Bulk {
   static constexpr size_t kCodeBytes = 2 * static_cast<size_t>(kTile) * DR;      // codes, sign bits: in x's place
   static constexpr size_t kSmem = kMatBytes + (kXBytes > kCodeBytes ? kXBytes : kCodeBytes);
   static constexpr int kPerLane = DR / 32;
+  // Resident CTAs per SM, as shared memory (50 KB at 64 coordinates, 98 KB at 128) and 128 to 255 registers allow.
+  static constexpr int kCtas = DR == 128 ? 2 : (DR == 96 ? 3 : 4);
 };
 
 // Word (j, i) of the matrix: groups of four coordinates exchanged with the row so that the transposing writes of a warp
@@ -477,9 +485,30 @@ __device__ __forceinline__ void bulk_chains(const float* __restrict__ mat, const
   }
 }
 
-template <int DR>
-__global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs a) {
+// Four vectors n0 .. of a warp, a lane its coordinates lane, lane + 32, ...: all loads in flight before the first use.
+template <int PL, typename T>
+__device__ __forceinline__ void load_four(const T* __restrict__ x, int64_t pitch, int64_t n0, int64_t n_vec, int d, int lane,
+                                          float (&xv)[4][PL]) {
+  T v[4][PL];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int t = 0; t < PL; ++t) {
+      const int j = lane + 32 * t;
+      v[u][t] = (n0 + u < n_vec && j < d) ? x[(n0 + u) * pitch + j] : T(0.f);
+    }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int t = 0; t < PL; ++t) xv[u][t] = static_cast<float>(v[u][t]);
+}
+
+// PAIR: both jobs of an append, by blockIdx.y.  (One job by itself reads its arguments at fixed addresses: 2 us of 37 at
+// 20000 vectors of 64 coordinates.)
+template <int DR, bool PAIR>
+__global__ void __launch_bounds__(kThreads, Bulk<DR>::kCtas) compress_bulk_kernel(ChainArgs args) {
   using B = Bulk<DR>;
+  const CompressArgs& a = args.job[PAIR ? blockIdx.y : 0];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float tab_s[2][16], cent_s[2][16], sgn_s[kMaxD];
   __shared__ uint32_t mask_words[kWarps];
@@ -520,14 +549,9 @@ __global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs
     // norm (sum of squares in fp64, rounded once), scale, stage transposed; a warp's vectors four at a time
     for (int u0 = 4 * warp; u0 < B::kTile; u0 += 4 * kWarps) {
       float xv[4][B::kPerLane];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int t = 0; t < B::kPerLane; ++t) {
-          const int j = lane + 32 * t;
-          const int64_t n = v0 + u0 + u;
-          xv[u][t] = (n < a.n_vec && j < d) ? load_float(a.x, a.x_dtype, n * a.x_pitch + j) : 0.f;
-        }
+      if (a.x_dtype == QKV_F32) load_four(static_cast<const float*>(a.x), a.x_pitch, v0 + u0, a.n_vec, d, lane, xv);
+      else if (a.x_dtype == QKV_BF16) load_four(static_cast<const __nv_bfloat16*>(a.x), a.x_pitch, v0 + u0, a.n_vec, d, lane, xv);
+      else load_four(static_cast<const __half*>(a.x), a.x_pitch, v0 + u0, a.n_vec, d, lane, xv);
       float norm[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -544,7 +568,8 @@ __global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs
             make_float4(xv[0][t] / norm[0], xv[1][t] / norm[1], xv[2][t] / norm[2], xv[3][t] / norm[3]);
       if (lane < 4) {
         const int64_t n = v0 + u0 + lane;
-        const int64_t row = n < a.n_vec ? map_row(a.rows, n) : -1;
+        const int64_t row = n < a.n_vec ? (PAIR ? chain_row(args, a, n) : map_row(a.rows, n)) : -1;
+        if (PAIR && row < 0 && n < a.n_vec && blockIdx.y == 0) atomicAdd(&g_rows_dropped, 1ull);
         row_s[u0 + lane] = row;
         if (row >= 0) a.norms[row] = lane == 0 ? norm[0] : (lane == 1 ? norm[1] : (lane == 2 ? norm[2] : norm[3]));
       }
@@ -557,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const int i = (c < 4 ? 4 * cx : DR / 2 + 4 * cx - 4) + c;
-        const int cls = cls_s[i], pos = slot_s[i];
+        const int cls = cls_s[i], pos = a.packed ? slot_s[i] : i;
         const float* tab = tab_s[cls];
         const float sgn = sgn_s[i];
 #pragma unroll
@@ -574,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs
       }
     }
     __syncthreads();
-    const bool whole16 = !mixed && (d & 15) == 0 &&
+    const bool whole16 = (d & 15) == 0 &&
         ((reinterpret_cast<uintptr_t>(a.codes) | reinterpret_cast<uintptr_t>(a.signs)) & 15u) == 0;
     if (!a.packed && whole16) {
       const int per_row = d >> 4;
@@ -590,7 +615,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs
         const int v = it / d, i = it - v * d;
         const int64_t row = row_s[v];
         if (row < 0) continue;
-        a.codes[row * d + i] = cs[v * DR + slot_s[i]];
+        a.codes[row * d + i] = cs[v * DR + i];
         if (with_signs) a.signs[row * d + i] = ss[v * DR + i];
       }
     } else {
@@ -610,7 +635,7 @@ __global__ void __launch_bounds__(kThreads, 2) compress_bulk_kernel(CompressArgs
 }
 
 template <int DR>
-__global__ void __launch_bounds__(kThreads, 2) decompress_bulk_kernel(DecompressArgs a) {
+__global__ void __launch_bounds__(kThreads, Bulk<DR>::kCtas) decompress_bulk_kernel(DecompressArgs a) {
   using B = Bulk<DR>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float tab_s[2][16], nrm_s[B::kTile];
@@ -639,14 +664,29 @@ __global__ void __launch_bounds__(kThreads, 2) decompress_bulk_kernel(Decompress
     const int64_t v0 = tile * B::kTile;
     for (int u0 = 4 * warp; u0 < B::kTile; u0 += 4 * kWarps) {
       float y[4][B::kPerLane];
+      int64_t row[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int64_t n = v0 + u0 + u;
-        const bool live = n < a.n_vec;
-        const int64_t row = live ? map_row(a.rows, n) : 0;
+        row[u] = n < a.n_vec ? (n < a.rows.seg_len ? a.rows.seg_off + n : map_row(a.rows, n)) : -1;     // (one segment: no division)
+        if (lane == u) nrm_s[u0 + u] = row[u] >= 0 ? a.norms[row[u]] : 0.f;
+      }
+      uint32_t c[4][B::kPerLane];                // codes of all four vectors before their look-ups
 #pragma unroll
-        for (int t = 0; t < B::kPerLane; ++t) y[u][t] = (live && lane + 32 * t < d) ? ch.value(a, tab_s, row, t, lane) : 0.f;
-        if (lane == u) nrm_s[u0 + u] = live ? a.norms[row] : 0.f;
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int t = 0; t < B::kPerLane; ++t) c[u][t] = (row[u] >= 0 && lane + 32 * t < d) ? ch.code(a, row[u], t, lane) : 0u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int t = 0; t < B::kPerLane; ++t)
+          y[u][t] = (row[u] >= 0 && lane + 32 * t < d) ? tab_s[ch.cls[t]][c[u][t] & 15u] : 0.f;
+      if (a.signs) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int t = 0; t < B::kPerLane; ++t)
+            if (row[u] >= 0 && lane + 32 * t < d) y[u][t] += ch.sign_term(a, ch.sign(a, row[u], t, lane), t);
       }
 #pragma unroll
       for (int t = 0; t < B::kPerLane; ++t)
@@ -696,8 +736,9 @@ void plan(int64_t n, int ctas_max, int& vt, int& ctas) {
   ctas = static_cast<int>(tiles < ctas_max ? tiles : ctas_max);
 }
 
-// From how many vectors on the bulk kernels are the faster ones: they need a CTA's worth of 64 vectors or more on most
-// SMs before their FMA rate counts.
+// From how many vectors (of both jobs) on the bulk kernels are the faster ones: they need a CTA's worth of 64 vectors or
+// more on most SMs before their FMA rate counts.  Append of 2 x 16384 vectors of 32 / 64 coordinates: 40 / 61 us in the
+// small kernel, 35 / 38 in bulk; of 2 x 4096 of 64, below the line: 19 against 25.
 template <int DR> constexpr int64_t bulk_from() { return static_cast<int64_t>(Bulk<DR>::kTile) * kNumSMs / 2; }
 
 template <typename K>
@@ -709,17 +750,16 @@ int set_smem(K kernel, size_t bytes) {
 template <int DR>
 int bulk_grid(int64_t n) {
   const int64_t tiles = (n + Bulk<DR>::kTile - 1) / Bulk<DR>::kTile;
-  return static_cast<int>(tiles < 2 * kNumSMs ? tiles : 2 * kNumSMs);
+  return static_cast<int>(tiles < Bulk<DR>::kCtas * kNumSMs ? tiles : Bulk<DR>::kCtas * kNumSMs);
 }
 
 template <int DR>
 int launch_compress_t(ChainArgs& args, cudaStream_t st) {
   const int jobs = args.job[1].n_vec > 0 ? 2 : 1;
-  const bool direct = args.records || args.block_table;       // destinations that the small kernel alone writes
-  if (args.job[0].n_vec >= bulk_from<DR>() && !direct) {
-    if (set_smem(compress_bulk_kernel<DR>, Bulk<DR>::kSmem)) return QKV_ELAUNCH;
-    for (int k = 0; k < jobs; ++k)
-      compress_bulk_kernel<DR><<<bulk_grid<DR>(args.job[k].n_vec), kThreads, Bulk<DR>::kSmem, st>>>(args.job[k]);
+  if (jobs * args.job[0].n_vec >= bulk_from<DR>() && !args.records) {      // (records: the small kernel alone writes them)
+    const auto kernel = jobs == 2 ? compress_bulk_kernel<DR, true> : compress_bulk_kernel<DR, false>;
+    if (set_smem(kernel, Bulk<DR>::kSmem)) return QKV_ELAUNCH;
+    kernel<<<dim3(bulk_grid<DR>(args.job[0].n_vec), jobs), kThreads, Bulk<DR>::kSmem, st>>>(args);
     return check_launch();
   }
   int ctas = 0;

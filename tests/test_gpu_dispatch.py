@@ -254,3 +254,24 @@ def test_a_backward_pass_through_an_op_is_refused():
     with torch.inference_mode():
         eng.append(torch.randn(1, 2, 3, 64, device=DEV), torch.randn(1, 2, 3, 64, device=DEV))
         assert eng.attention(torch.randn(1, 4, 1, 64, device=DEV)).shape == (1, 4, 1, 64)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,n", [(128, 5001), (96, 6007), (80, 6001), (64, 9473), (32, 18999), (20, 18945)])
+def test_bulk_chain_kernels_equal_the_small_ones(D, n, dtype, monkeypatch):
+    """The same fp32 chains in the kernel of many vectors and, in pieces of 1000, in that of few: the same bytes, norms
+    and values, for every layout."""
+    monkeypatch.setenv("QUASHKV_B200_CUDA_CORE_ROTATION", "1")
+    x = _outliers(torch.Generator(device=DEV).manual_seed(D), (n, D), dtype)
+    mixed = qk.MixedPrecisionMSEQuantizer(D, 3, 2, D // 4 + 1, seed=42, device=DEV)
+    mixed.calibrate(x[:500].float())
+    mse, ip = qk.MSEQuantizer(D, 4, seed=42, device=DEV), qk.InnerProductQuantizer(D, 3, seed=42, device=DEV)
+    for fn in (mse.compress, mse.compress_packed, ip.compress, ip.compress_packed,
+               lambda v: mixed.compress(v, packed=False), lambda v: mixed.compress(v, packed=True)):
+        whole, parts = fn(x), [fn(x[i:i + 1000]) for i in range(0, n, 1000)]
+        for i, got in enumerate(whole):
+            assert torch.equal(got, torch.cat([p[i] for p in parts]))
+    for codes, norms, fn in ((*mse.compress(x), mse.decompress), (*mse.compress_packed(x), mse.decompress_packed),
+                             (*mixed.compress(x, packed=True), lambda c, s: mixed.decompress(c, s, packed=True)),
+                             (*mixed.compress(x, packed=False), lambda c, s: mixed.decompress(c, s, packed=False))):
+        assert torch.equal(fn(codes, norms), torch.cat([fn(codes[i:i + 1000], norms[i:i + 1000]) for i in range(0, n, 1000)]))
