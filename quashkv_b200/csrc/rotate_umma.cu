@@ -130,7 +130,9 @@ __device__ __forceinline__ UmmaSmem carve_umma(unsigned char* raw) {
 // stream position n' and every 32-column block belongs to one table; this needs the number of
 // outlier channels to be a multiple of 32 (otherwise the CTA returns at once and the CUDA-core
 // kernel, launched behind it with the same test inverted, does the work).
-template <int BITS, bool IP, int NT, int BITS1 = 0>
+// BYTES: one byte per coordinate instead of packed rows.  (A template parameter: as a test in the epilogue it cost the packed
+// forms two registers too many, 2 % of their time.)
+template <int BITS, bool IP, int NT, int BITS1 = 0, bool BYTES = false>
 __global__ void __launch_bounds__(kUThreads, 1) compress_umma_kernel(CompressArgs a) {
   constexpr bool MIXED = BITS1 != 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kUThreads, 1) compress_umma_kernel(CompressArg
         for (int b = 0; b < (1 << bits_c) - 1; ++b) code += z > bnd_s[cls][b] ? 1u : 0u;
         const int64_t row = map_row(a.rows, n);
         const uint32_t diff = code ^ old_code;
-        if (!MIXED && !a.packed) {                 // one byte per coordinate
+        if (BYTES) {
           if (diff) a.codes[row * kRD + col] = static_cast<uint8_t>(code);
           if (IP) {
             const uint32_t sign = ((z - cent_s[code]) * sgn_s[col] >= 0.f) ? 1u : 0u;
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(kUThreads, 1) compress_umma_kernel(CompressArg
     }
     // unflagged coordinates: sign = residual >= 0 exclusive-or S < 0 (a zero residual is always flagged)
     const uint32_t sign_word = IP ? ((~(__brev(R) ^ smask) & ~fmask) | fval) : 0u;
-    if (!MIXED && !a.packed) {
+    if (BYTES) {
       // One byte per coordinate: a thread holds 32 neighbouring bytes of a row, a whole sector, and four codes leave
       // the packed words with one extraction and two spreads.
       if (live) {
@@ -640,21 +642,23 @@ bool compress_umma_ok(const CompressArgs& a) {
          (a.x_pitch & 7) == 0 && (al & 15u) == 0;
 }
 
-template <int BITS, bool IP, int NT>
+template <int BITS, bool IP, int NT, bool BYTES>
 static int launch_compress_umma_n(const CompressArgs& a, cudaStream_t st) {
   constexpr size_t smem = umma_smem_bytes<NT>();
-  if (cudaFuncSetAttribute(compress_umma_kernel<BITS, IP, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(compress_umma_kernel<BITS, IP, NT, 0, BYTES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem)) != cudaSuccess)
     return QKV_ELAUNCH;
   const int64_t tiles = (a.n_vec + kUTile - 1) / kUTile;
   const int grid = static_cast<int>(tiles < kNumSMs ? tiles : kNumSMs);
-  compress_umma_kernel<BITS, IP, NT><<<grid, kUThreads, smem, st>>>(a);
+  compress_umma_kernel<BITS, IP, NT, 0, BYTES><<<grid, kUThreads, smem, st>>>(a);
   return check_launch();
 }
 
 template <int BITS, bool IP>
 static int launch_compress_umma_t(const CompressArgs& a, cudaStream_t st) {
-  return a.x_dtype == QKV_BF16 ? launch_compress_umma_n<BITS, IP, 1>(a, st) : launch_compress_umma_n<BITS, IP, 3>(a, st);
+  if (a.packed)
+    return a.x_dtype == QKV_BF16 ? launch_compress_umma_n<BITS, IP, 1, false>(a, st) : launch_compress_umma_n<BITS, IP, 3, false>(a, st);
+  return a.x_dtype == QKV_BF16 ? launch_compress_umma_n<BITS, IP, 1, true>(a, st) : launch_compress_umma_n<BITS, IP, 3, true>(a, st);
 }
 
 template <int B0, int B1>
