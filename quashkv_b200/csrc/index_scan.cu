@@ -240,11 +240,11 @@ __global__ void topk_merge_kernel(const float* __restrict__ in_s, const int64_t*
             out_s + static_cast<int64_t>(m) * k_out, out_i + static_cast<int64_t>(m) * k_out, lane);
 }
 
-// Long candidate lists (few queries, many slices): one CTA of 32 warps per query.  A warp takes its share of the list
+// Long candidate lists (few queries, many slices): one CTA of eight to 32 warps per query.  A warp takes its share of the list
 // eight entries per lane at a time into registers, all loads in flight, together with the k best so far (from shared
-// memory), and picks k in rank order with one exchange over the warp each; the first warp then does the same with the
-// warps' lists.  Bound by latency: the kernel before it walked over the list in memory once per result, which took
-// 72 us for 7700 entries and k = 10.
+// memory), and picks k in rank order with one exchange over the warp each; the first warp then merges the sorted
+// lists, a lane holding the head of each, with one exchange per result.  Bound by latency: the kernel before it walked
+// over the list in memory once per result.
 constexpr int kWideWarps = 32;
 constexpr int kWideNew = 8, kWideOld = QKV_INDEX_MAX_K / 32;
 
@@ -301,6 +301,39 @@ __device__ __forceinline__ void warp_topk_registers(const float* s, const int64_
   __syncwarp();
 }
 
+// The k best of up to 32 lists of k entries in rank order (shared memory; missing entries last), by one warp, to global
+// memory; equal (score, id) pairs of different lists count once.
+__device__ __forceinline__ void merge_sorted_lists(const float* s, const int64_t* ids, int lists, int k, float* os, int64_t* oi,
+                                                   int lane) {
+  s += lane * k;
+  ids += lane * k;
+  int at = lane < lists ? 0 : k;
+  float head = at < k ? s[0] : -INFINITY;
+  int64_t head_i = at < k ? ids[0] : -1;
+  int r = 0;
+  for (; r < k; ++r) {
+    float w = head;
+    int64_t wi = head_i;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float w2 = __shfl_xor_sync(QKV_FULL_MASK, w, o);
+      const int64_t i2 = __shfl_xor_sync(QKV_FULL_MASK, wi, o);
+      if (i2 >= 0 && (wi < 0 || ranks_before(w2, i2, w, wi))) { w = w2; wi = i2; }
+    }
+    wi = __shfl_sync(QKV_FULL_MASK, wi, 0);               // (an undefined score orders no two lanes alike)
+    w = __shfl_sync(QKV_FULL_MASK, w, 0);
+    if (wi < 0) break;
+    if (lane == 0) { os[r] = w; oi[r] = wi; }
+    if (w != w) { ++r; break; }                           // nothing ranks after an undefined score
+    if (head_i == wi && head == w) {
+      ++at;
+      head = at < k ? s[at] : -INFINITY;
+      head_i = at < k ? ids[at] : -1;
+    }
+  }
+  for (int e = r + lane; e < k; e += 32) { os[e] = -INFINITY; oi[e] = -1; }
+}
+
 __global__ void __launch_bounds__(kWideWarps * 32)
 topk_merge_wide_kernel(const float* __restrict__ in_s, const int64_t* __restrict__ in_i, int M, int64_t n_cand,
                        int k_out, float* __restrict__ out_s, int64_t* __restrict__ out_i,
@@ -310,30 +343,30 @@ topk_merge_wide_kernel(const float* __restrict__ in_s, const int64_t* __restrict
   const int mc = blockIdx.x;
   if (mc >= (qlist ? qlist[M] : M)) return;                                 // CTA-uniform
   const int m = qlist ? qlist[mc] : mc;
-  int64_t* part_i = reinterpret_cast<int64_t*>(smem_raw);                   // [warps + 1][k]
-  float* part_s = reinterpret_cast<float*>(part_i + (kWideWarps + 1) * k_out);
-  const int64_t chunk = (n_cand + kWideWarps - 1) / kWideWarps;
+  int64_t* part_i = reinterpret_cast<int64_t*>(smem_raw);                   // [warps][k]
+  const int warps = static_cast<int>(blockDim.x >> 5);
+  float* part_s = reinterpret_cast<float*>(part_i + warps * k_out);
+  const int64_t chunk = (n_cand + warps - 1) / warps;
   const int64_t lo = warp * chunk, hi = lo + chunk < n_cand ? lo + chunk : n_cand;
   warp_topk_registers(in_s + static_cast<int64_t>(mc) * n_cand + lo, in_i + static_cast<int64_t>(mc) * n_cand + lo,
                       hi > lo ? hi - lo : 0, k_out, part_s + warp * k_out, part_i + warp * k_out, lane);
   __syncthreads();
-  if (warp == 0) {
-    float* fs = part_s + kWideWarps * k_out;
-    int64_t* fi = part_i + kWideWarps * k_out;
-    warp_topk_registers(part_s, part_i, kWideWarps * k_out, k_out, fs, fi, lane);
-    for (int r = lane; r < k_out; r += 32) {
-      out_s[static_cast<int64_t>(m) * k_out + r] = fs[r];
-      out_i[static_cast<int64_t>(m) * k_out + r] = fi[r];
-    }
-  }
+  if (warp == 0)
+    merge_sorted_lists(part_s, part_i, warps, k_out, out_s + static_cast<int64_t>(m) * k_out, out_i + static_cast<int64_t>(m) * k_out,
+                       lane);
 }
 
 static void launch_topk_merge(const float* in_s, const int64_t* in_i, int M, int64_t n_cand, int k_out,
                               float* out_s, int64_t* out_i, const int* qlist, cudaStream_t st) {
   if (n_cand >= 2048 && k_out <= QKV_INDEX_MAX_K) {
-    const size_t smem = static_cast<size_t>(kWideWarps + 1) * k_out * 12;
+    // Few queries: all 32 warps, for latency.  More of them than SMs: as many as have a full load of 256 entries each, since
+    // the picks of a list take the same time whatever its length (512 lists of 2048, k = 10: 70 us with 32 warps, 41 with
+    // a walk over memory by eight, 33 with eight of these).
+    const int64_t full = (n_cand + 32 * kWideNew - 1) / (32 * kWideNew);
+    const int warps = M <= kNumSMs || full > kWideWarps ? kWideWarps : (full < 8 ? 8 : static_cast<int>(full));
+    const size_t smem = static_cast<size_t>(warps) * k_out * 12;
     if (smem > 49152) cudaFuncSetAttribute(topk_merge_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    topk_merge_wide_kernel<<<M, kWideWarps * 32, smem, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i, qlist);
+    topk_merge_wide_kernel<<<M, warps * 32, smem, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i, qlist);
   } else {
     const int warps = 4;
     topk_merge_kernel<<<(M + warps - 1) / warps, warps * 32, 0, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i,

@@ -275,3 +275,24 @@ def test_bulk_chain_kernels_equal_the_small_ones(D, n, dtype, monkeypatch):
                              (*mixed.compress(x, packed=True), lambda c, s: mixed.decompress(c, s, packed=True)),
                              (*mixed.compress(x, packed=False), lambda c, s: mixed.decompress(c, s, packed=False))):
         assert torch.equal(fn(codes, norms), torch.cat([fn(codes[i:i + 1000], norms[i:i + 1000]) for i in range(0, n, 1000)]))
+
+
+@pytest.mark.parametrize("k", [1, 7, 10, 31, 40, 100, 128])
+@pytest.mark.parametrize("M,n", [(1, 2048), (3, 2049), (5, 8191), (2, 20000), (149, 2048), (200, 3333), (150, 8300)])
+def test_merge_of_long_candidate_lists(M, n, k):
+    """Every count of warps and loads: ties (few distinct scores), pairs that stand in the list twice (they count once),
+    missing entries, and fewer candidates than results; rank order is by score, then by the smaller id."""
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    scores = torch.randint(-40, 40, (M, n), generator=g, device=DEV).float() / 8
+    scores[:, ::2] += torch.randn(M, (n + 1) // 2, generator=g, device=DEV)
+    ids = torch.randint(0, 3 * n, (M, n), generator=g, device=DEV)
+    ids[:, 1::7] = ids[:, :-1:7][:, :ids[:, 1::7].shape[1]]                    # the same pair next to itself ...
+    scores[:, 1::7] = scores[:, :-1:7][:, :scores[:, 1::7].shape[1]]
+    ids[:, n // 2 + 5], scores[:, n // 2 + 5] = ids[:, 3], scores[:, 3]          # ... and in another warp's share
+    ids[:, ::11] = -1
+    ids[-1, 5:] = -1                                                           # hardly any candidates at all
+    got_s, got_i = qk.ops.topk_merge(scores, ids, k)
+    for m in {0, M // 2, M - 1}:
+        pairs = sorted({(-s, i) for s, i in zip(scores[m].tolist(), ids[m].tolist()) if i >= 0})[:k]
+        want = [(-s, i) for s, i in pairs] + [(float("-inf"), -1)] * (k - len(pairs))
+        assert list(zip(got_s[m].tolist(), got_i[m].tolist())) == want
