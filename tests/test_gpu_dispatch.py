@@ -14,21 +14,31 @@ DEV = "cuda"
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n", [1, 3, 129, 6143, 6144, 6271, 9473])
-def test_unpacked_codes_equal_the_packed_ones(n, dtype):
+def test_unpacked_codes_equal_the_packed_ones(n, dtype, monkeypatch):
     """One byte per coordinate and packed rows, at every width, on both sides of the size from which the tensor-core
-    kernel runs: whole numbers, so they are the same."""
+    kernel runs, against the fp32 chain: whole numbers, so they are the same."""
     x = torch.randn(n, 128, generator=torch.Generator().manual_seed(n)).to(dtype).to(DEV)
+
+    def chain(fn):
+        monkeypatch.setenv("QUASHKV_B200_CUDA_CORE_ROTATION", "1")
+        out = fn(x)
+        monkeypatch.delenv("QUASHKV_B200_CUDA_CORE_ROTATION")
+        return out
+
     for bits in (1, 2, 3, 4):
         q = qk.MSEQuantizer(128, bits, seed=42, device=DEV)
         codes, norms = q.compress(x)
         packed, norms_p = q.compress_packed(x)
         assert torch.equal(qk.unpack_bits(packed, bits, 128), codes) and torch.equal(norms, norms_p)
+        want, norms_w = chain(q.compress)
+        assert torch.equal(codes, want) and torch.equal(norms, norms_w)
     for bits in (2, 3, 4):
         q = qk.InnerProductQuantizer(128, bits, seed=42, device=DEV)
         codes, signs, norms = q.compress(x)
         packed, packed_s, norms_p = q.compress_packed(x)
         assert torch.equal(qk.unpack_bits(packed, bits - 1, 128), codes) and torch.equal(norms, norms_p)
         assert torch.equal(qk.unpack_bits(packed_s, 1, 128), signs)
+        assert all(torch.equal(a, b) for a, b in zip((codes, signs, norms), chain(q.compress)))
 
 
 def _outliers(g, shape, dtype):
@@ -45,6 +55,8 @@ def _outliers(g, shape, dtype):
     (321, 130, 2, True, torch.bfloat16),          # rows of two heads in one row tile, a ragged end everywhere
     (1, 1, 160, False, torch.float32),            # a single token
     (640, 512, 1, True, torch.bfloat16),          # whole row tiles, heaviest first
+    (1024, 512, 4, True, torch.bfloat16),         # ... of several heads, each with its own order; sixteen token tiles
+    (1300, 1024, 8, True, torch.float32),         # ... over an older cache of ragged length
 ])
 def test_prefill_kernels_match_the_decode_kernels(D, kb, vb, n, q_len, G, causal, dtype, monkeypatch):
     """The same call through the kernels of long and of short query blocks.  Both hold fp32 (about 5e-7 from 64-bit

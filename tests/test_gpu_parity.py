@@ -186,12 +186,6 @@ def test_tensor_core_rotation_equals_cuda_core_rotation(golden, monkeypatch):
             slow_ip = ops.compress_ip(xd, Pi, bnd, cent, S, bits, packed=True)
             rec_slow = ops.decompress(fast[0], fast[1], Pi, cent, bits, packed=True, d=128)
             monkeypatch.delenv("QUASHKV_B200_CUDA_CORE_ROTATION")
-            monkeypatch.setenv("QUASHKV_B200_NO_TCGEN05", "1")       # bf16 input: mma.sync instead of tcgen05
-            mid = ops.compress_mse(xd, Pi, bnd, bits, packed=True)
-            mid_ip = ops.compress_ip(xd, Pi, bnd, cent, S, bits, packed=True)
-            monkeypatch.delenv("QUASHKV_B200_NO_TCGEN05")
-            assert torch.equal(mid[0], slow[0]) and torch.equal(mid_ip[0], slow_ip[0])
-            assert torch.equal(mid_ip[1], slow_ip[1]) and torch.equal(mid[1], slow[1])
             n_code = int((fast[0] != slow[0]).sum()) + int((fast_ip[0] != slow_ip[0]).sum())
             n_sign = int((fast_ip[1] != slow_ip[1]).sum())
             print(f"[ties] tensor-core vs CUDA-core rotation, {dtype}, {bits} bits: {n_code} code bytes, "
@@ -305,7 +299,8 @@ def test_tcgen05_rotation_edge_shapes(golden, monkeypatch):
     Pi, S = t(c["Pi_d128_s42"]).to(DEV), t(c["S_d128_s42"]).to(DEV)
     bnd, cent = t(c["bnd_d128_b2"]).to(DEV), t(c["cent_d128_b2"]).to(DEV)
     gen = torch.Generator().manual_seed(5)
-    x = torch.randn(3 * 1000 + 77, 128, generator=gen)
+    n = 2500                    # three segments of it, and the ragged batch, are past the size from which compress uses tcgen05
+    x = torch.randn(3 * n + 77, 128, generator=gen)
 
     def both(fn):
         fast = fn()
@@ -322,25 +317,25 @@ def test_tcgen05_rotation_edge_shapes(golden, monkeypatch):
         a, b = both(lambda: ops.decompress(mse, nrm, Pi, cent, 2, signs=qjl, S=S, qjl_scale=0.0123, packed=True,
                                            d=128, out_dtype=dt))
         assert rel_l2(a, b) < tol, f"IP decompress {dt}: {rel_l2(a, b)}"
-    # engine planes: 3 segments of capacity 1280, 1000 live rows each, written in place at offset 100
-    K = torch.randn(1, 3, 1000, 128, generator=gen).to(torch.bfloat16).to(DEV)
-    V = torch.randn(1, 3, 1000, 128, generator=gen).to(torch.bfloat16).to(DEV)
+    # engine planes: 3 segments of capacity 2816, 2500 live rows each, written in place at offset 100
+    K = torch.randn(1, 3, n, 128, generator=gen).to(torch.bfloat16).to(DEV)
+    V = torch.randn(1, 3, n, 128, generator=gen).to(torch.bfloat16).to(DEV)
     vb, vc = t(c["bnd_d128_b3"]).to(DEV), t(c["cent_d128_b3"]).to(DEV)
 
     def planes():
-        p = {"k_codes": torch.zeros(3, 1280, 32, dtype=torch.uint8, device=DEV),
-             "k_signs": torch.zeros(3, 1280, 16, dtype=torch.uint8, device=DEV),
-             "k_norms": torch.zeros(3, 1280, device=DEV),
-             "v_codes": torch.zeros(3, 1280, 48, dtype=torch.uint8, device=DEV),
-             "v_norms": torch.zeros(3, 1280, device=DEV)}
+        p = {"k_codes": torch.zeros(3, 2816, 32, dtype=torch.uint8, device=DEV),
+             "k_signs": torch.zeros(3, 2816, 16, dtype=torch.uint8, device=DEV),
+             "k_norms": torch.zeros(3, 2816, device=DEV),
+             "v_codes": torch.zeros(3, 2816, 48, dtype=torch.uint8, device=DEV),
+             "v_norms": torch.zeros(3, 2816, device=DEV)}
         ops.append_kv(K, V, Pi, bnd, cent, S, 2, vb, 3, p["k_codes"], p["k_signs"], p["k_norms"], p["v_codes"],
                       p["v_norms"], 100)
         return p
     pf, ps = both(planes)
     for name in pf:
         assert torch.equal(pf[name], ps[name]), name
-    a, b = both(lambda: ops.decompress_rows(pf["v_codes"], pf["v_norms"], Pi, vc, 3, 128, 3, 1000, 1280, 100))
-    assert a.shape == (3000, 128) and rel_l2(a, b) < 2e-6
+    a, b = both(lambda: ops.decompress_rows(pf["v_codes"], pf["v_norms"], Pi, vc, 3, 128, 3, n, 2816, 100))
+    assert a.shape == (3 * n, 128) and rel_l2(a, b) < 2e-6
     from quashkv_b200 import _lib
     assert _lib.lib().qkv_tensor_core_timeouts() == TIMEOUTS[0]
 
@@ -1147,7 +1142,8 @@ def test_paged_decode_steps_and_pool_exhaustion():
 def test_paged_append_with_device_tables_matches_host_bookkeeping(D, bs):
     """A serving engine that owns the page allocation hands over its device block table and start lengths:
     the slots are computed on the device and the pool ends up byte-identical to the one filled through the
-    pool's own (host) bookkeeping; attention over the caller's tables gives the same output."""
+    pool's own (host) bookkeeping, every token where the table says, counted here, it is; attention over the caller's
+    tables gives the same output."""
     from quashkv_b200.integrations.vllm_backend import QuashKVPageConfig, QuashKVPagedCache
     Hkv, n = 2, 3
     cfg = QuashKVPageConfig(block_size=bs)
@@ -1166,6 +1162,21 @@ def test_paged_append_with_device_tables_matches_host_bookkeeping(D, bs):
     for name in host.planes:
         assert torch.equal(host.planes[name], dev.planes[name]), name
     table, lens, mx = host.block_table(ids)
+    # the rows of every sequence, token by token from its pages, against a compression of the same tokens by themselves
+    e = host.engine
+    want = dict(zip(("k_codes", "k_signs", "k_norms"), e.key_quantizer.compress_packed(K)))
+    want.update(zip(("v_codes", "v_norms"), e.value_quantizer.compress_packed(V)))
+    for name in want:
+        if host.tiled:
+            slots = torch.tensor([(int(table[i, p // bs]) * Hkv + h) * bs + p % bs
+                                  for i in range(n) for h in range(Hkv) for p in range(50)], device=DEV)
+            rows = dict(zip(("k_codes", "k_signs", "k_norms", "v_codes", "v_norms"),
+                            ops.untile_rows(dev.planes["records"], slots.numel(), 1, 0, 0, slots)))[name]
+            assert torch.equal(rows.reshape(want[name].shape), want[name]), name
+        else:
+            for i in range(n):
+                for p in range(50):
+                    assert torch.equal(dev.planes[name][int(table[i, p // bs]), :, p % bs], want[name][i, :, p]), (name, i, p)
     Q = torch.randn(n, Hkv * 4, 1, D, generator=g).to(DEV)
     assert torch.equal(host.attention(ids, Q), dev.attention_with_tables(Q, table, lens, mx))
 
@@ -1384,6 +1395,14 @@ def test_tensor_core_wait_that_runs_out_falls_back_to_exact_arithmetic(monkeypat
     TIMEOUTS[0] = after
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+    monkeypatch.setenv("QUASHKV_B200_TEST_DROP_MMA", "1")    # one byte per coordinate leaves through an epilogue of its own
+    got_bytes = q.compress(x)
+    torch.cuda.synchronize()
+    monkeypatch.delenv("QUASHKV_B200_TEST_DROP_MMA")
+    assert _lib.lib().qkv_tensor_core_timeouts() > after
+    TIMEOUTS[0] = after = _lib.lib().qkv_tensor_core_timeouts()
+    assert torch.equal(got_bytes[0], ops.unpack(want[0], 2, 128)) and torch.equal(got_bytes[1], ops.unpack(want[1], 1, 128))
+    assert torch.equal(got_bytes[2], want[2])
     again = q.compress_packed(x)                             # and the library is as before afterwards
     assert torch.equal(again[0], want[0]) and _lib.lib().qkv_tensor_core_timeouts() == after
 
