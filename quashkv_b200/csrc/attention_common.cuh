@@ -159,8 +159,8 @@ int launch_prefill(const AttnArgs& a, const void* q, int q_dtype, int key_bits, 
                    float scale, void* workspace, cudaStream_t st);
 unsigned int bulk_copy_timeouts();        // bounded waits on a record copy that ran out (device-wide counter)
 
-// Look-up tables of the tensor-core path, built by one CTA of 128 threads.  For each table the scale
-// s in [1,2) (512 candidates, 4 per thread) is chosen that makes the largest relative fp16 rounding
+// Look-up tables of the tensor-core path, built by one CTA.  For each table the scale s in [1,2) (512 candidates, shared
+// out among its threads) is chosen that makes the largest relative fp16 rounding
 // error of s*c_i smallest, so the systematic error of the fp16 operands drops well below 2^-12.
 // tables[0..1] key centroids as fp16 pairs, [2..3] value low bytes, [4..5] value high bytes,
 // [6] 1/key scale, [7] 1/value scale (floats), [8..9] the four value magnitudes (entries 4..7 of the

@@ -45,45 +45,6 @@ __device__ __forceinline__ uint32_t read_field(const uint8_t* row, int bitpos, i
   return (v >> sh) & ((1u << w) - 1u);
 }
 
-// Pack 32 codes (one per lane) of width W into W little-endian words: stream bit p of the
-// group is bit (p % W) of the code held by lane p / W.  Returns word `lane` on lanes < W.
-template <int W>
-__device__ __forceinline__ uint32_t pack32_fixed(uint32_t code, int lane) {
-  uint32_t mine = 0;
-#pragma unroll
-  for (int k = 0; k < W; ++k) {
-    const int p = 32 * k + lane;
-    const uint32_t c = __shfl_sync(QKV_FULL_MASK, code, p / W);
-    const uint32_t word = __ballot_sync(QKV_FULL_MASK, (c >> (p % W)) & 1u);
-    if (lane == k) mine = word;
-  }
-  return mine;
-}
-
-__device__ __forceinline__ uint32_t pack32(uint32_t code, int w, int lane) {
-  switch (w) {
-    case 1: return pack32_fixed<1>(code, lane);
-    case 2: return pack32_fixed<2>(code, lane);
-    case 3: return pack32_fixed<3>(code, lane);
-    default: return pack32_fixed<4>(code, lane);
-  }
-}
-
-// Store the words produced by pack32 at row + byte_off, never touching bytes >= byte_end.
-__device__ __forceinline__ void store_packed_words(uint32_t mine, int w, uint8_t* row, int byte_off,
-                                                   int byte_end, int lane) {
-  if (lane >= w) return;
-  const int off = byte_off + 4 * lane;
-  uint8_t* p = row + off;
-  if (off + 4 <= byte_end && (reinterpret_cast<uintptr_t>(p) & 3u) == 0) {
-    *reinterpret_cast<uint32_t*>(p) = mine;
-  } else {
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-      if (off + b < byte_end) p[b] = static_cast<uint8_t>(mine >> (8 * b));
-  }
-}
-
 // q_rot = q @ Pi^T per row; writes [row][0][d] = q_rot*scale and
 // [row][1][d] = qjl_scale*scale*|q_rot|*S.  Defined in attention.cu.
 int launch_rotate_queries(const void* q, int q_dtype, int64_t rows, int d, const float* Pi, const float* S,

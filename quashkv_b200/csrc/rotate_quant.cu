@@ -23,14 +23,8 @@ static bool cuda_core_only() {
   return e && e[0] == '1';
 }
 
-// QUASHKV_B200_NO_TCGEN05=1 keeps the rotation off the tcgen05 kernels (for A/B checks).
-static bool no_tcgen05() {
-  const char* e = getenv("QUASHKV_B200_NO_TCGEN05");
-  return e && e[0] == '1';
-}
-
 bool compress_prefers_chain(const CompressArgs& a) {
-  return !compress_umma_ok(a) || cuda_core_only() || no_tcgen05();
+  return !compress_umma_ok(a) || cuda_core_only();
 }
 
 static int run_compress(const CompressArgs& a, cudaStream_t st) {
@@ -49,7 +43,7 @@ static int run_compress(const CompressArgs& a, cudaStream_t st) {
 }
 
 static int run_decompress(DecompressArgs& a, cudaStream_t st) {
-  if (decompress_umma_ok(a) && !cuda_core_only() && !no_tcgen05()) {
+  if (decompress_umma_ok(a) && !cuda_core_only()) {
     const int rc = launch_decompress_umma(a, st);
     if (rc || a.mode != MODE_MIXED) return rc;
     a.skip_block_aligned = 1;        // as above: outlier counts that are no multiple of 32

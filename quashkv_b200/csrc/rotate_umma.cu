@@ -17,7 +17,7 @@
 // packed row.  A coordinate whose bucket holds a decision boundary is classified exactly from a register copy
 // (tensor memory is re-read only for threads with several such coordinates); coordinates within kRecheckEps of a
 // boundary go to a per-warp queue and are recomputed with the sequential fp32 FMA chain, exactly as in the
-// mma.sync kernel, so the bytes are identical to the CUDA-core kernel's.  The queues are emptied by all warps
+// fp32 chain kernels, so the bytes are identical to the CUDA-core kernel's.  The queues are emptied by all warps
 // together (a flag out of the tile barrier), and the products of a tile are issued one at a time between the
 // phases of the loop, because the issuing thread is held for about as long as its MMAs execute.
 //
