@@ -22,8 +22,8 @@
 // queries, tables and weights to fp16 once as well: TERMS = 1).  Error against 64-bit results: with TERMS = 2 0.71 of the
 // fp32 kernel's on average over 34 shapes, 0.93 at the worst of them; with TERMS = 1 that of the kernels it stands beside.
 //
-// Measured (before: the decode kernels): 8 x 1024 causal tokens, 32 / 4 heads of 64, 8609 -> 500 us; 2 x 4096, 32 / 8 heads
-// of 128 at 3/3 bits, 3016 -> 1000 us.  Bound by the softmax warps' chain (tensor memory reads, 1.8 instructions a cycle);
+// Measured, append and attention (before: the decode kernels): 8 x 1024 causal tokens, 32 / 4 heads of 64, 8609 -> 443 us;
+// 2 x 4096, 32 / 8 heads of 128 at 3/3 bits, 3013 -> 993 us (attention alone 385 and 880).  Bound by the softmax warps' chain (tensor memory reads, 1.8 instructions a cycle);
 // the tensor pipe is 20 % busy.
 //
 // Every wait is bounded; one that runs out is counted and ends the use of the tensor core in its CTA, whose rows are then
