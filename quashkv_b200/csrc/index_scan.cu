@@ -359,11 +359,11 @@ topk_merge_wide_kernel(const float* __restrict__ in_s, const int64_t* __restrict
 static void launch_topk_merge(const float* in_s, const int64_t* in_i, int M, int64_t n_cand, int k_out,
                               float* out_s, int64_t* out_i, const int* qlist, cudaStream_t st) {
   if (n_cand >= 2048 && k_out <= QKV_INDEX_MAX_K) {
-    // Few queries: all 32 warps, for latency.  More of them than SMs: as many as have a full load of 256 entries each, since
-    // the picks of a list take the same time whatever its length (512 lists of 2048, k = 10: 70 us with 32 warps, 41 with
-    // a walk over memory by eight, 33 with eight of these).
+    // As many warps as have a full load of 256 entries each: the picks of a list take the same time whatever its length, and
+    // warps that share a scheduler wait for one another (one list of 2048, k = 40: 66 us with 32 warps, 51 with eight; 512
+    // of them, k = 10: 70 and 33, a walk over memory by eight warps 41).
     const int64_t full = (n_cand + 32 * kWideNew - 1) / (32 * kWideNew);
-    const int warps = M <= kNumSMs || full > kWideWarps ? kWideWarps : (full < 8 ? 8 : static_cast<int>(full));
+    const int warps = full > kWideWarps ? kWideWarps : (full < 8 ? 8 : static_cast<int>(full));
     const size_t smem = static_cast<size_t>(warps) * k_out * 12;
     if (smem > 49152) cudaFuncSetAttribute(topk_merge_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     topk_merge_wide_kernel<<<M, warps * 32, smem, st>>>(in_s, in_i, M, n_cand, k_out, out_s, out_i, qlist);
